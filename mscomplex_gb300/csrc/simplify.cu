@@ -14,14 +14,17 @@
 // C++ standard library the reference is built with.  Persistence |f2 - f1| is
 // precomputed per heap entry; the comparator is "d1 > d2" (a min-heap on d).
 //
-// The replay is sequential by nature and runs on one thread of one block.
-// Multisets (critical_point::asc / des, std::multiset<uint>) are run-length
-// encoded sorted arrays in a device pool; they grow by reallocation inside it.
-// Every loop is bounded: the pass stops with ST_SIMPLIFY_LIMIT when the
-// operation budget or a pool runs out, leaving the complex unmodified.
+// The replay is sequential by nature: one warp of one block makes the heap
+// operations and graph edits in order, and its lanes share the work inside
+// each of them (struct Simp; warp_graph.cuh).  Multisets
+// (critical_point::asc / des, std::multiset<uint>) are run-length encoded
+// sorted arrays in a device pool; they grow by reallocation inside it.  Every
+// loop is bounded: the pass stops with ST_SIMPLIFY_LIMIT when the operation
+// budget or a pool runs out, leaving the complex unmodified.
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 #include "msc_graph.cuh"
+#include "warp_graph.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -93,11 +96,14 @@ __host__ __device__ inline uint32_t stop_bits(float max_persistence, double tres
 struct SimpArgs {
   Graph G;            // the complex as a mutable graph (msc_graph.cuh)
   const float *fn;
-  uint32_t *meta;     // per critical point: its index with the entry bits (k_simp_prep)
-  HeapEnt *heap;
+  uint32_t *meta;     // per critical point: its index with the entry bits (k_simp_meta); its pair's order (k_unsimplify)
+  float *hkey;        // the heap in global memory, keys and pairs apart, entries 1 .. heap_cap
+  uint2 *hab;
   unsigned long long heap_cap;
   HeapEnt *resub;     // resubmit list (capacity heap_cap), whole entries
   uint2 *canc;        // cancellation list (capacity ncp)
+  uint32_t ncanc;     // its length, and whether it holds a pair that was not connected (for k_unsimplify)
+  bool loose;
   int rx0, ry0, rx1, ry1;  // m_rect of the complex (cell coordinates)
   double tresh;
   unsigned long long *stats;  // [0] pushes [1] pops [2] cancels [3] ops [4] status
@@ -108,277 +114,475 @@ struct SimpArgs {
   unsigned long long ninit;
 };
 
-// The top HEAP_TOP entries of the heap (its first 14 levels, which every pop
-// walks) live in shared memory; the rest in global memory.  Same layout and
-// the same operations, only the storage of those indices differs.
-constexpr unsigned long long HEAP_TOP = (1u << 14) - 1;
-constexpr size_t HEAP_TOP_BYTES = sizeof(HeapEnt) * HEAP_TOP;
+// The heap's first TL levels, which every pop walks, live in shared memory,
+// the rest in global memory; both hold keys and (a, b) pairs in separate
+// arrays indexed from 1 (entry k has the children 2k and 2k + 1), so that one
+// aligned 8-byte load gets both children's keys.
+constexpr int TOP_LEVELS = 14, TOP_LEVELS_BATCH = 13;
+// The block's warps: the first replays the heap, the others edit the lists
+// of cancelled pairs, each with shared memory for a long list's edit.
+constexpr int SIMP_WARPS = 4, HELPERS = SIMP_WARPS - 1;
+__host__ __device__ constexpr uint32_t edit_runs(int levels) { return levels == TOP_LEVELS ? 1024 : 512; }
+__host__ __device__ constexpr size_t top_bytes(int levels) {
+  return ((sizeof(float) + sizeof(uint2)) << levels) + sizeof(uint2) * HELPERS * edit_runs(levels);
+}
+// The state the warps share: the pair being cancelled, and whether to stop.
+// The first warp starts the helpers through barrier BAR_GO and waits for them
+// through BAR_DONE; each is passed by every thread of the block once per
+// cancellation (BAR_GO once more at the end, with stop set).
+struct SimpShared {
+  TeamState team;
+  WarpGraph::Pair pair;
+  int stop;
+};
+constexpr int BAR_GO = 1, BAR_DONE = 2;
+__device__ __forceinline__ void bar_arrive(int b) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(b), "r"(32 * SIMP_WARPS) : "memory");
+}
+__device__ __forceinline__ void bar_wait(int b) {
+  asm volatile("bar.sync %0, %1;" ::"r"(b), "r"(32 * SIMP_WARPS) : "memory");
+}
+constexpr unsigned long long HEAP_MAX = 0xFFFFFFE0ull;  // entries: 32-bit indices, one lane per level in a push
 
+// The replay by one warp.  What bounds it is the latency of each dependent
+// step, so the lanes take the steps of one heap operation together:
+//   * pop: the hole's path to the leaves depends on the keys alone.  Each lane
+//     compares the two children of one node of the 5-level subtree under the
+//     hole; a ballot of the choices tells every lane whether its node lies on
+//     the path (its ancestors' choices, a mask of constants per lane), so one
+//     load and two ballots replace five dependent loads, and the path's entries
+//     move up together;
+//   * push: one lane per ancestor compares its key; a ballot gives the climb;
+//   * a burst of pushes (the first pushes, the resubmit list, new edges): 32
+//     at a time, the entries that stay where they are pushed (their parent is
+//     not larger) are stored at once.
+// A cancellation's list edits go to the block's other warps (help): they are
+// chains of dependent loads of lists no one has touched for long, and until
+// the next pair is classified the heap needs none of them, so they run beside
+// the pushes of the new edges and of the resubmit list and the next pop.
+// On the 256x256 noisy field at 5% (35,000 pops, 1,520 cancellations) one
+// thread took 2,150 cycles a pop, 710 a push and 23,000 a cancellation, 74 ms
+// in all; here a pop takes 750, a push 225 and a cancellation waits 550 for
+// its edits, 24 ms in all.
 struct Simp {
   SimpArgs A;
-  unsigned long long nheap = 0, nres = 0, ncanc = 0;
-  unsigned long long n_push = 0, n_pop = 0;  // heap operations (stats[0], stats[1] at the end)
-  HeapEnt *top = nullptr;         // shared-memory part of the heap (null: all in global memory)
-  unsigned long long ntop = 0;    // indices below ntop are in `top`
+  WarpGraph W;
+  float *skey;
+  uint2 *sab;
+  uint32_t ntop;                  // entries below it are in shared memory (a power of two)
+  uint32_t nheap = 0, nres = 0, ncanc = 0;
+  unsigned long long n_pop = 0;   // heap operations (the pushes: the pops and what is left)
+  bool ordered = false;           // no key is NaN (all values finite)
+  bool loose = false;             // a pair that was not connected is on the cancellation list
+  // this lane's node of the 5-level subtree under entry h is h * mul + add (lane 31: none), its
+  // ancestors among the lanes are anc, and those of them in need must choose the right child
+  uint32_t mul, add, anc, need;
 
-  __host__ __device__ __forceinline__ HeapEnt &H(unsigned long long i) { return i < ntop ? top[i] : A.heap[i]; }
-  // L1 prefetch of the global part of heap[lo..hi], one request per 128-byte line
-  __host__ __device__ __forceinline__ void prefetch_heap(unsigned long long lo, unsigned long long hi) {
-#ifdef __CUDA_ARCH__
-    if (lo < ntop) lo = ntop;
-    if (hi >= A.heap_cap) hi = A.heap_cap - 1;
-    if (lo > hi) return;
-    const char *p = reinterpret_cast<const char *>(A.heap + lo), *e = reinterpret_cast<const char *>(A.heap + hi + 1);
-    for (p = reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)127); p < e; p += 128)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-#else
-    (void)lo; (void)hi;
-#endif
+  SimpShared *sh;
+  bool pending = false;           // the helpers are at work
+
+  __device__ Simp(const SimpArgs &a, void *smem, int levels, SimpShared *shared) : A(a), sh(shared) {
+    W.G = a.G;
+    W.lane = threadIdx.x & 31;
+    ntop = 1u << levels;
+    sab = reinterpret_cast<uint2 *>(smem);
+    skey = reinterpret_cast<float *>(sab + ntop);
+    const uint32_t i = (uint32_t)W.lane + 1;  // 1-based node of the subtree
+    const int ll = 31 - __clz(i);
+    mul = 1u << ll;
+    add = i - mul;
+    anc = need = 0;
+    for (int s = 1; s <= ll; ++s) {
+      anc |= 1u << ((i >> s) - 1);
+      if ((i >> (s - 1)) & 1u) need |= 1u << ((i >> s) - 1);
+    }
+    if (W.lane == 31) { mul = 0; add = 0xFFFFFFFFu; }
+    W.stage = nullptr;
+    W.nstage = 0;
   }
-  // before a burst of m pushes at the end: the lines of the three ancestor
-  // levels above the positions they take, and of the entries themselves
-  __host__ __device__ __forceinline__ void prefetch_pushes(const HeapEnt *src, unsigned long long m) {
-#ifdef __CUDA_ARCH__
-    if (m == 0) return;
-    const unsigned long long n0 = nheap, n1 = nheap + m;
-    for (int k = 1; k <= 3; ++k) prefetch_heap(((n0 + 1) >> k) - 1, ((n1 + 1) >> k) - 1);
-    const char *p = reinterpret_cast<const char *>(src), *e = reinterpret_cast<const char *>(src + m);
-    for (p = reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)127); p < e; p += 128)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-#else
-    (void)src; (void)m;
-#endif
+  // waits for the helpers' edits
+  __device__ __forceinline__ void settle() {
+    if (!pending) return;
+    pending = false;
+    bar_wait(BAR_DONE);
+    if (sh->team.fail) W.G.fail = true;
+    W.G.ops += sh->team.ops;
+    __syncwarp();
+    if (W.lane == 0) sh->team.ops = 0;
+    __syncwarp();
+  }
+  __device__ __forceinline__ float key_at(uint32_t k) const { return k < ntop ? skey[k] : A.hkey[k]; }
+  __device__ __forceinline__ void put(uint32_t k, float d, uint2 ab) {
+    if (k < ntop) { skey[k] = d; sab[k] = ab; }
+    else { A.hkey[k] = d; A.hab[k] = ab; }
   }
 
-  // ---- heap (binary heap of the standard library, comparator d1 > d2) ----
-  __host__ __device__ __forceinline__ static bool comp(const HeapEnt &x, const HeapEnt &y) { return x.d > y.d; }
-  // __push_heap from position hole up to the root: the hole climbs while its
-  // parent is larger (comparator d1 > d2) -- in global memory while the hole
-  // is there, then in shared memory with 32-bit indices
-  __host__ __device__ void push_at(unsigned long long hole, HeapEnt val) {
-    while (hole >= ntop && hole > 0) {
-      const unsigned long long parent = (hole - 1) / 2;
-      const HeapEnt pe = H(parent);
-      if (!comp(pe, val)) { H(hole) = val; return; }
-      H(hole) = pe;
-      hole = parent;
+  // __push_heap from entry k (comparator d1 > d2): the entry climbs while its
+  // parent is larger.  Lane l holds the ancestor l + 1 levels up and, where
+  // every lane below it climbs, fills the place l levels up.
+  template <bool TOP>  // TOP: entry k, and so all of its ancestors, in shared memory
+  __device__ __forceinline__ void push_at(uint32_t k, float d, uint2 ab) {
+    const uint32_t to = k >> W.lane, p = to >> 1;
+    float pk;
+    uint2 pab;
+    if (TOP || p < ntop) {  // (entry 0 is never used)
+      pk = skey[p];
+      pab = sab[p];
+    } else {
+      pk = A.hkey[p];
+      pab = A.hab[p];
     }
-    if (hole >= ntop) { H(hole) = val; return; }  // the root itself is in global memory (no shared part)
-    uint32_t h = (uint32_t)hole;
-    while (h > 0) {
-      const uint32_t parent = (h - 1) >> 1;
-      if (!(top[parent].d > val.d)) break;
-      top[h] = top[parent];
-      h = parent;
+    const bool climbs = p != 0 && pk > d;
+    const unsigned up = __ballot_sync(FULL_WARP, climbs);
+    if ((~up & W.lt()) == 0) {
+      pk = climbs ? pk : d;
+      pab = climbs ? pab : ab;
+      if (TOP) { skey[to] = pk; sab[to] = pab; }
+      else put(to, pk, pab);
     }
-    top[h] = val;
+    __syncwarp();
   }
-  __host__ __device__ void push_ent(const HeapEnt &x) {
-    if (nheap >= A.heap_cap) { A.G.fail = true; return; }
-    push_at(nheap, x);
-    ++nheap;
-    ++n_push;
+  // The lanes of `mask` push their entries, in lane order.  An entry whose
+  // parent is not larger stays at its own place and changes no other; the
+  // climbs of the others only lower the keys of their ancestors (where the
+  // keys are ordered), so it stays there whether they come before or after it.
+  template <bool TOP>
+  __device__ __forceinline__ void push_lanes_t(unsigned mask, uint32_t cnt, float d, uint2 ab) {
+    const uint32_t k = nheap + 1 + __popc(mask & W.lt());
+    unsigned todo = mask;
+    if (ordered && nheap >= 32) {  // every parent is an older entry
+      const bool on = (mask >> W.lane) & 1u;
+      const uint32_t p = on ? k >> 1 : 0;
+      const bool climbs = on && (TOP ? skey[p] : key_at(p)) > d;
+      if (on && !climbs) {
+        if (TOP) { skey[k] = d; sab[k] = ab; }
+        else put(k, d, ab);
+      }
+      todo = __ballot_sync(FULL_WARP, climbs);
+    }
+    nheap += cnt;
+    // the next entry is on its way while one climbs
+    uint32_t nk = 0;
+    float ndv = 0.0f;
+    uint2 nab = make_uint2(0, 0);
+    auto next = [&]() {
+      const int s = (__ffs(todo) - 1) & 31;
+      nk = __shfl_sync(FULL_WARP, k, s);
+      ndv = __shfl_sync(FULL_WARP, d, s);
+      nab = make_uint2(__shfl_sync(FULL_WARP, ab.x, s), __shfl_sync(FULL_WARP, ab.y, s));
+    };
+    next();
+    while (todo) {
+      const uint32_t ck = nk;
+      const float cd = ndv;
+      const uint2 cab = nab;
+      todo &= todo - 1;
+      next();
+      push_at<TOP>(ck, cd, cab);
+    }
   }
-  // a new pair: its two values and its two entry words from independent loads
-  __host__ __device__ void push(uint32_t a, uint32_t b) {
-    const float fa = A.fn[a], fb = A.fn[b];
-    const uint32_t ma = A.meta[a], mb = A.meta[b];
-    push_ent(HeapEnt{fabsf(fsub_rn(fb, fa)), ma, mb});
+  __device__ __forceinline__ void push_lanes(unsigned mask, float d, uint2 ab) {
+    __syncwarp();
+    const uint32_t cnt = __popc(mask);
+    if ((unsigned long long)nheap + cnt > A.heap_cap) { W.G.fail = true; return; }
+    if (nheap + cnt < ntop) push_lanes_t<true>(mask, cnt, d, ab);
+    else push_lanes_t<false>(mask, cnt, d, ab);
   }
+  __device__ __forceinline__ static unsigned first_lanes(unsigned long long n) {
+    return n >= 32 ? FULL_WARP : (1u << (unsigned)n) - 1u;
+  }
+  __device__ __forceinline__ void push_entries(const HeapEnt *src, unsigned long long n) {
+    __syncwarp();
+    HeapEnt nx{0.0f, 0, 0};
+    if ((unsigned)W.lane < n) nx = src[W.lane];
+    for (unsigned long long q = 0; q < n && !W.G.fail; q += 32) {
+      const HeapEnt e = nx;
+      if (q + 32 + W.lane < n) nx = src[q + 32 + W.lane];  // the next 32 on their way
+      push_lanes(first_lanes(n - q), e.d, make_uint2(e.a, e.b));
+    }
+  }
+  // pushes (d, a) for every occurrence of a value in p[0..n) but `skip`, in
+  // order: the value is the pair's second point with `other` the first
+  // (second = true), or the other way round
+  __device__ __forceinline__ void push_edges(const uint2 *p, uint32_t n, uint32_t skip, uint32_t other, bool second) {
+    const float fo = A.fn[other];
+    const uint32_t mo = A.meta[other];
+    for (uint32_t i0 = 0; i0 < n && !W.G.fail; i0 += 32) {
+      uint2 r = make_uint2(skip, 0);
+      if (i0 + W.lane < n) r = p[i0 + W.lane];
+      const bool on = r.x != skip;
+      const uint32_t at = on ? r.x : other;
+      const uint32_t mr = A.meta[at];
+      const float fr = A.fn[at];
+      const float d = fabsf(second ? fsub_rn(fr, fo) : fsub_rn(fo, fr));
+      const uint2 ab = second ? make_uint2(mo, mr) : make_uint2(mr, mo);
+      const unsigned many = __ballot_sync(FULL_WARP, on && r.y > 1), all = __ballot_sync(FULL_WARP, on);
+      if (!many) {
+        push_lanes(all, d, ab);
+        continue;
+      }
+      for (unsigned todo = all; todo && !W.G.fail; todo &= todo - 1) {  // copies: one value after the other
+        const int s = __ffs(todo) - 1;
+        const uint32_t c = __shfl_sync(FULL_WARP, r.y, s);
+        const float ds = __shfl_sync(FULL_WARP, d, s);
+        const uint2 as = make_uint2(__shfl_sync(FULL_WARP, ab.x, s), __shfl_sync(FULL_WARP, ab.y, s));
+        for (uint32_t q = 0; q < c && !W.G.fail; q += 32) push_lanes(first_lanes(c - q), ds, as);
+      }
+    }
+  }
+
   // pop_heap + pop_back: libstdc++'s __adjust_heap moves the hole from the
   // root to a leaf along the smaller children (the right one unless the left
   // is strictly smaller), then sifts the last element up from that leaf.  The
   // sift-up restores every path entry below the place where the last element
-  // lands, so stopping the descent there -- at the first chosen child larger
-  // than the last element -- leaves the same heap with fewer steps.
-  //
-  // The path does not depend on the last element, so the shared-memory part
-  // is chosen first from the keys alone (while the last element, often in
-  // global memory, is still on its way), then shifted up to the stop; in
-  // global memory both children and all four grandchildren of the hole are
-  // loaded together, two levels per round trip.
-  __host__ __device__ HeapEnt pop() {
+  // lands, so the hole stops there -- at the first chosen child larger than
+  // the last element -- which leaves the same heap with fewer moves.  The
+  // popped entry is on top before the call.
+  __device__ __forceinline__ void pop() {
     ++n_pop;
-    HeapEnt first = H(0);
-    const unsigned long long len = nheap - 1;
-    --nheap;
-    if (len == 0) return first;
-    const HeapEnt val = H(len);
-    // the next pops' last elements are the entries below this one: keep
-    // their lines on their way into L1
-    if (len >= ntop + 16) prefetch_heap(len - 16, len - 16);
-    unsigned long long hole = 0;
-    // shared-memory levels: the path while both children are in `top`, two
-    // levels per step (children and grandchildren keys loaded together),
-    // kept in registers (fixed-size arrays indexed by unrolled constants)
-    constexpr int PMAX = 14;  // HEAP_TOP holds 14 levels
-    uint32_t path[PMAX];
-    float pkey[PMAX];
-    int np = 0;
-    {
-      // 32-bit indices: every index here is below ntop (at most HEAP_TOP); len
-      // is clamped, which keeps each comparison with it exact
-      const uint32_t nt = (uint32_t)ntop, ln = len > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)len;
-      uint32_t h = 0;
-#pragma unroll
-      for (int q = 0; q < PMAX; q += 2) {
-        const uint32_t l = 2 * h + 1;
-        if (l >= ln || l + 1 >= nt) break;
-        const uint32_t ll = 2 * l + 1, rl = ll + 2;  // first child of l and of l + 1
-        const bool g_ok = rl + 1 < nt;              // all four grandchildren in `top`
-        const float dl = top[l].d, dr = l + 1 < ln ? top[l + 1].d : 0.0f;
-        float g0 = 0, g1 = 0, g2 = 0, g3 = 0;
-        if (g_ok) { g0 = top[ll].d; g1 = top[ll + 1].d; g2 = top[rl].d; g3 = top[rl + 1].d; }
-        const bool right = l + 1 < ln && !(dr > dl);
-        const uint32_t c = right ? l + 1 : l;
-        path[q] = c;
-        pkey[q] = right ? dr : dl;
-        np = q + 1;
-        h = c;
-        if (q + 1 >= PMAX || !g_ok) break;
-        const uint32_t l2 = 2 * c + 1;
-        if (l2 >= ln) break;
-        const float el = right ? g2 : g0, er = right ? g3 : g1;
-        const bool right2 = l2 + 1 < ln && !(er > el);
-        const uint32_t c2 = right2 ? l2 + 1 : l2;
-        path[q + 1] = c2;
-        pkey[q + 1] = right2 ? er : el;
-        np = q + 2;
-        h = c2;
+    if (nheap < ntop) pop_t<true>();
+    else pop_t<false>();
+  }
+  template <bool TOP>  // TOP: the whole heap in shared memory
+  __device__ __forceinline__ void pop_t() {
+    const uint32_t last = nheap, len = --nheap;  // entries 1 .. len remain
+    if (len == 0) return;
+    float vd;
+    uint2 vab;
+    if (TOP) {
+      vd = skey[last];
+      vab = sab[last];
+    } else {
+      vd = A.hkey[last];
+      vab = A.hab[last];
+      // the next pops' last elements: their lines on their way into L1
+      if (len >= ntop + 32) {
+        if (W.lane == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(A.hkey + len - 32));
+        if (W.lane == 1) asm volatile("prefetch.global.L1 [%0];" ::"l"(A.hab + len - 16));
       }
     }
-    int stop = np;
+    // shared-memory levels: the path from the keys alone, five levels a round
+    constexpr int R = 3;
+    const uint32_t lim = TOP ? len : ntop - 1;
+    const uint32_t half = lim >> 1, half1 = (lim - 1) >> 1;  // the last entries with a left / a right child there
+    float ck[R];
+    uint32_t nd[R], h = 1;
+    uint2 mv[R];
+    bool on[R];
 #pragma unroll
-    for (int i = PMAX - 1; i >= 0; --i)
-      if (i < np && pkey[i] > val.d) stop = i;
-    {
-      // the path's entries first (independent loads), then each one level up
-      HeapEnt mv[PMAX];
-#pragma unroll
-      for (int i = 0; i < PMAX; ++i)
-        if (i < stop) mv[i] = top[path[i]];
-      uint32_t hs = 0;  // the hole while it is in shared memory (32-bit)
-#pragma unroll
-      for (int i = 0; i < PMAX; ++i) {
-        if (i >= stop) break;
-        top[hs] = mv[i];
-        hs = path[i];
+    for (int r = 0; r < R; ++r) {
+      on[r] = false;
+      nd[r] = 0;
+      ck[r] = 0.0f;
+      if (lim >= (2u << (5 * r))) {  // (known early: the path's own end is found without branches)
+        nd[r] = h * mul + add;
+        const bool has = nd[r] <= half;
+        float2 kk = make_float2(0.0f, 0.0f);
+        if (has) kk = reinterpret_cast<const float2 *>(skey)[nd[r]];
+        const bool right = nd[r] <= half1 && !(kk.y > kk.x);
+        const unsigned D = __ballot_sync(FULL_WARP, right);
+        on[r] = has && ((D ^ need) & anc) == 0;
+        const uint32_t child = 2 * nd[r] + (right ? 1u : 0u);
+        ck[r] = right ? kk.y : kk.x;
+        if (on[r]) mv[r] = sab[child];
+        h = __reduce_max_sync(FULL_WARP, on[r] ? child : h);  // the path's last child
       }
-      hole = hs;
     }
-    if (stop < np) {  // the last element lands in shared memory
-      top[hole] = val;
-      return first;
+    // the first path node whose chosen child is larger than the last element;
+    // the entries above it move up
+    uint32_t place = 0xFFFFFFFFu;
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r)
+      if (on[r] && ck[r] > vd) place = nd[r];
+    place = __reduce_min_sync(FULL_WARP, place);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (on[r] && nd[r] < place) { skey[nd[r]] = ck[r]; sab[nd[r]] = mv[r]; }
+    __syncwarp();
+    if (TOP) {  // (every lane stores the same)
+      place = place == 0xFFFFFFFFu ? h : place;
+      skey[place] = vd;
+      sab[place] = vab;
+    } else {
+      if (place == 0xFFFFFFFFu) place = pop_global(h, len, vd);
+      if (W.lane == 0) put(place, vd, vab);
     }
-    // global levels (and the step from the last shared-memory node), two at a time
-    for (;;) {
-      const unsigned long long l = 2 * hole + 1;
-      if (l >= len) break;
-      const bool has_r = l + 1 < len;
-      const unsigned long long ll = 2 * l + 1, rl = 2 * (l + 1) + 1;
-      const HeapEnt L = H(l), R = has_r ? H(l + 1) : L;
-      HeapEnt g[4];
-      g[0] = ll < len ? H(ll) : L;
-      g[1] = ll + 1 < len ? H(ll + 1) : L;
-      g[2] = rl < len ? H(rl) : L;
-      g[3] = rl + 1 < len ? H(rl + 1) : L;
-      const bool right = has_r && !(R.d > L.d);
-      const unsigned long long c = right ? l + 1 : l;
-      const HeapEnt hc = right ? R : L;
-      if (hc.d > val.d) break;
-      H(hole) = hc;
-      hole = c;
-      // the next level from the loaded grandchildren
-      const unsigned long long l2 = 2 * c + 1;
-      if (l2 >= len) break;
-      const HeapEnt L2 = right ? g[2] : g[0], R2 = right ? g[3] : g[1];
-      const bool right2 = l2 + 1 < len && !(R2.d > L2.d);
-      const HeapEnt hc2 = right2 ? R2 : L2;
-      if (hc2.d > val.d) break;
-      H(hole) = hc2;
-      hole = right2 ? l2 + 1 : l2;
+    __syncwarp();
+  }
+  // the levels in global memory, five a round trip; the place of the last element
+  __device__ __forceinline__ uint32_t pop_global(uint32_t h, uint32_t len, float vd) {
+    const uint32_t half = len >> 1, half1 = (len - 1) >> 1;
+    while (h <= half) {
+      const unsigned long long nd = (unsigned long long)h * mul + add;
+      const bool has = nd <= half;
+      float2 kk = make_float2(0.0f, 0.0f);
+      if (has) kk = reinterpret_cast<const float2 *>(A.hkey)[nd];
+      const bool right = nd <= half1 && !(kk.y > kk.x);
+      const unsigned D = __ballot_sync(FULL_WARP, right);
+      bool on = has && ((D ^ need) & anc) == 0;
+      const uint32_t child = 2 * (uint32_t)nd + (right ? 1u : 0u);
+      const float ck = right ? kk.y : kk.x;
+      const uint32_t place = __reduce_min_sync(FULL_WARP, on && ck > vd ? (uint32_t)nd : 0xFFFFFFFFu);
+      h = __reduce_max_sync(FULL_WARP, on ? child : 0u);
+      on = on && nd < place;
+      uint2 mv;
+      if (on) mv = A.hab[child];
+      __syncwarp();
+      if (on) put((uint32_t)nd, ck, mv);
+      __syncwarp();
+      if (place != 0xFFFFFFFFu) return place;
     }
-    H(hole) = val;
-    return first;
+    return h;
   }
 
-  // simplify (grid_mscomplex.cpp:384-512) followed by un_simplify (:514-526)
-  __host__ __device__ void run() {
-    Graph &G = A.G;
+  // simplify (grid_mscomplex.cpp:384-512)
+  __device__ __forceinline__ void run() {
+    Graph &G = W.G;
     const uint32_t n = G.ncp;
+    const bool lead = W.lane == 0;
     // (:396-428) the strangulation marks and the entries of the first pushes
     // come from k_simp_prep; the value range and the pushes, in the
     // reference's order, here
     float max_val = 1.17549435e-38f;  // std::numeric_limits<float>::min(), as in the reference (:399)
     float min_val = 3.40282347e+38f;
-    for (uint32_t i = 0; i < n; ++i) {
+    for (uint32_t i = W.lane; i < n; i += 32) {
       const float f = A.fn[i];
       max_val = (max_val < f) ? f : max_val;  // std::max
       min_val = (f < min_val) ? f : min_val;  // std::min
     }
-    for (unsigned long long q = 0; q < A.ninit && !G.fail; ++q) push_ent(A.init[q]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float a = __shfl_xor_sync(FULL_WARP, max_val, o), b = __shfl_xor_sync(FULL_WARP, min_val, o);
+      max_val = (max_val < a) ? a : max_val;
+      min_val = (b < min_val) ? b : min_val;
+    }
+    ordered = max_val <= 3.40282347e+38f && min_val >= -3.40282347e+38f;
+    push_entries(A.init, A.ninit);
+    if (G.fail) nheap = 0;  // (nothing is popped; the pass has failed)
     const float max_persistence = fsub_rn(max_val, min_val);
     const uint32_t stop_at = stop_bits(max_persistence, A.tresh);
-    while (nheap != 0 && !G.fail) {
-      if (!G.tick()) break;
+    const uint32_t ncl = n ? n - 1 : 0;
+    float rd = 0.0f;  // resubmitted entries past the last full 32, one per lane
+    uint2 rab = make_uint2(0, 0);
+    while (nheap != 0) {
+      ++G.ops;
       // the entry on top and its pair's dynamic state (three independent
       // loads), issued before the pop's descent so that they arrive during it
-      const HeapEnt top0 = H(0);
-      uint32_t w1 = top0.a, w2 = top0.b;
-      if (ent_dim(w2) == 1) { uint32_t t = w1; w1 = w2; w2 = t; }
+      const float ed = skey[1];
+      const uint2 eab = sab[1];
+      const bool turn = ent_dim(eab.y) == 1;
+      const uint32_t w1 = turn ? eab.y : eab.x, w2 = turn ? eab.x : eab.y;
       const uint32_t v1 = ent_idx(w1), v2 = ent_idx(w2);
-      const bool inside = v1 < n && v2 < n;
       const int cp2_dim = ent_dim(w2);
-      const uint8_t f1 = inside ? G.flags[v1] : 0, f2 = inside ? G.flags[v2] : 0;
-      const uint32_t tot2 = inside ? G.L.total[2 * v2 + cp2_dim / 2] : 0;
-      HeapEnt e = pop();
-      if (float_bits(e.d) >= stop_at) break;  // (double)e.d / max_persistence > tresh
-      if (!inside) { A.stats[4] |= ST_INVARIANT; continue; }  // a list entry outside the complex
-      if ((f1 & F_CANCELLED) || (f2 & F_CANCELLED)) continue;
-      const bool b1 = ent_boundary(w1), b2 = ent_boundary(w2);
-      if (b1 && !b2) continue;
-      if (!b1 && b2) continue;
-      const bool strang = f1 & F_STRANG;
-      if (strang && tot2 != 1) {
-        if (nres >= A.heap_cap) { G.fail = true; break; }
-        A.resub[nres++] = e;
+      const uint32_t u1 = min(v1, ncl), u2 = min(v2, ncl);
+      uint32_t f1 = 0, f2 = 0, tot2 = 0;
+      uint2 dsc = make_uint2(0, 0);
+      auto state = [&]() {
+        f1 = G.flags[u1];
+        f2 = G.flags[u2];
+        tot2 = G.L.total[2 * u2 + cp2_dim / 2];
+        // should the pair be cancelled: its lists' places and lengths, one word pair per lane
+        dsc = reinterpret_cast<const uint2 *>((W.lane & 1) ? G.L.nrun : G.L.off)[(W.lane & 2) ? u2 : u1];
+      };
+      if (!pending) state();
+      __syncwarp();  // every lane has read the top
+      pop();
+      if (pending) {
+        settle();
+        if (G.fail) break;
+        state();
+      }
+      const bool b1 = ent_boundary(w1), b2 = ent_boundary(w2), strang = f1 & F_STRANG;
+      const bool stop = G.ops > G.max_ops || float_bits(ed) >= stop_at;  // (double)d / max_persistence > tresh
+      const bool inside = v1 == u1 && v2 == u2;
+      const bool skip = ((f1 | f2) & F_CANCELLED) || b1 != b2;
+      const bool again = strang && tot2 != 1;
+      if (!stop && inside && (skip || again)) {  // most pops
+        const bool mine = !skip && (uint32_t)W.lane == (nres & 31u);
+        rd = mine ? ed : rd;
+        rab = mine ? eab : rab;
+        nres += skip ? 0u : 1u;
+        if (!skip && (nres & 31u) == 0) {
+          if (nres > A.heap_cap) { G.fail = true; break; }
+          A.resub[nres - 32 + W.lane] = HeapEnt{rd, rab.x, rab.y};
+        }
+        continue;
+      }
+      if (stop) {
+        if (G.ops > G.max_ops) {  // the budget ends before this pop
+          G.fail = true;
+          --n_pop;
+          ++nheap;
+        }
+        break;
+      }
+      if (!inside) {  // a list entry outside the complex
+        if (lead) A.stats[4] |= ST_INVARIANT;
         continue;
       }
       if (strang && b1) continue;
-      uint32_t cp0 = v1, cp1 = v2;
-      bool connected = G.cancel_pairs(cp0, cp1);
-      if (G.fail) break;
-      G.flags[v1] |= F_BCANCEL;
-      G.flags[v2] |= F_BCANCEL;
-      G.pair_idx[v1] = v2;
-      G.pair_idx[v2] = v1;
+      // (an asc list holds points of the next dimension only)
+      uint2 pl[2], nr[2];  // of v1, v2
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        pl[q] = make_uint2(__shfl_sync(FULL_WARP, dsc.x, 2 * q), __shfl_sync(FULL_WARP, dsc.y, 2 * q));
+        nr[q] = make_uint2(__shfl_sync(FULL_WARP, dsc.x, 2 * q + 1), __shfl_sync(FULL_WARP, dsc.y, 2 * q + 1));
+      }
+      WarpGraph::Pair pr = cp2_dim == 0 ? WarpGraph::Pair{pl[1], pl[0], nr[1], nr[0], v2, v1}
+                                        : WarpGraph::Pair{pl[0], pl[1], nr[0], nr[1], v1, v2};
+      const bool connected = W.orient(pr);
       if (ncanc >= n) { G.fail = true; break; }
-      A.canc[ncanc++] = make_uint2(ent_idx(e.a), ent_idx(e.b));
-      if (connected) {  // new edges (d, a) in the reference's order
-        const uint32_t la0 = 2 * cp0, ld1 = 2 * cp1 + 1;
-        for (uint32_t i = 0; i < G.L.nrun[la0] && !G.fail; ++i) {
-          uint2 ra = G.runs(la0)[i];
-          if (ra.x == cp1) continue;
-          for (uint32_t ca = 0; ca < ra.y && !G.fail; ++ca)
-            for (uint32_t j = 0; j < G.L.nrun[ld1] && !G.fail; ++j) {
-              uint2 rd = G.runs(ld1)[j];
-              if (rd.x == cp0) continue;
-              for (uint32_t cd = 0; cd < rd.y && !G.fail; ++cd) push(rd.x, ra.x);
-            }
+      if (lead) {
+        if (connected) sh->pair = pr;
+        G.pair_idx[v1] = v2;
+        G.pair_idx[v2] = v1;
+        A.canc[ncanc] = connected ? make_uint2(pr.cp0, pr.cp1) : make_uint2(ent_idx(eab.x), ent_idx(eab.y));
+        if (!connected) {
+          G.flags[v1] |= F_BCANCEL;
+          G.flags[v2] |= F_BCANCEL;
         }
       }
-      prefetch_pushes(A.resub, nres);
-      for (unsigned long long i = 0; i < nres && !G.fail; ++i) push_ent(A.resub[i]);
+      ++ncanc;
+      loose |= !connected;
+      if (connected) {
+        W.close(pr, F_BCANCEL);
+        __syncwarp();
+        bar_arrive(BAR_GO);
+        pending = true;
+      }
+      __syncwarp();
+      if (connected) {  // new edges (d, a), a in asc(cp0) \ {cp1}, d in des(cp1) \ {cp0}, in the reference's order
+        const uint32_t cp0 = pr.cp0, cp1 = pr.cp1, na = pr.n0.x, nd = pr.n1.y;
+        const uint2 *pa = G.L.pool + pr.o0.x, *pd = G.L.pool + pr.o1.y;
+        uint2 r0 = make_uint2(cp0, 0), r1 = r0;  // des(cp1), when short
+        if (nd > 0) r0 = pd[0];
+        if (nd > 1) r1 = pd[1];
+        const uint2 one = r0.x != cp0 ? r0 : r1;
+        if (nd <= 2 && (r0.x == cp0 || r1.x == cp0) && (one.x == cp0 || one.y == 1)) {  // one d, or none
+          if (one.x != cp0) push_edges(pa, na, cp1, one.x, true);
+        } else {
+          for (uint32_t i = 0; i < na && !G.fail; ++i) {
+            const uint2 ra = pa[i];
+            if (ra.x == cp1) continue;
+            for (uint32_t ca = 0; ca < ra.y && !G.fail; ++ca) push_edges(pd, nd, cp0, ra.x, false);
+          }
+        }
+      }
+      if (!G.fail) {
+        push_entries(A.resub, nres & ~31u);
+        if (!G.fail && (nres & 31u)) push_lanes(first_lanes(nres & 31u), rd, rab);
+      }
+      if (G.fail) break;
       nres = 0;
     }
-    A.stats[0] = n_push;
-    A.stats[1] = n_pop;
-    A.stats[2] = ncanc;
-    if (G.fail) return;
-    for (unsigned long long k = ncanc; k-- > 0;) {
-      uint2 c = A.canc[k];
-      if (!G.uncancel_pairs(c.x, c.y)) { A.stats[4] |= ST_INVARIANT; return; }
-      if (G.fail) return;
+    settle();
+    if (G.ops > G.max_ops) G.fail = true;
+    if (lead) {
+      A.stats[0] = n_pop + nheap;
+      A.stats[1] = n_pop;
+      A.stats[2] = ncanc;
     }
   }
 };
@@ -417,16 +621,167 @@ __global__ void k_simp_prep(SimpArgs *args) {
   }
 }
 
-__global__ void k_simplify(SimpArgs a) {
-  extern __shared__ HeapEnt heap_top[];
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  Simp s;
-  s.A = a;
-  s.top = heap_top;
-  s.ntop = HEAP_TOP;
+// A helper warp: the list edits of every cancelled pair, until told to stop.
+__device__ __forceinline__ void help(const SimpArgs &a, SimpShared *sh, uint2 *stage, uint32_t runs) {
+  const int who = (int)(threadIdx.x >> 5) - 1;
+  WarpGraph W;
+  W.G = a.G;
+  W.lane = threadIdx.x & 31;
+  W.stage = stage + (size_t)who * runs;
+  W.nstage = runs;
+  W.G.tmp_cap = a.G.tmp_cap / HELPERS;
+  W.G.tmp = a.G.tmp + (size_t)who * W.G.tmp_cap;
+  W.G.max_ops = ~0ull;  // (the first warp keeps the budget)
+  W.team = &sh->team;
+  for (;;) {
+    bar_wait(BAR_GO);
+    if (sh->stop) return;
+    W.G.ops = 0;
+    W.edit_neighbours(sh->pair, who, HELPERS);
+    if (W.lane == 0) {
+      if (W.G.fail) sh->team.fail = 1;
+      atomicAdd(&sh->team.ops, W.G.ops);
+    }
+    __syncwarp();
+    bar_arrive(BAR_DONE);
+  }
+}
+
+// one complex per block
+__global__ void __launch_bounds__(32 * SIMP_WARPS, 2) k_simplify(SimpArgs *args, int n, int levels) {
+  extern __shared__ __align__(16) unsigned char heap_top[];
+  __shared__ SimpShared sh;
+  if (blockIdx.x >= (unsigned)n) return;
+  const SimpArgs a = args[blockIdx.x];
+  if (threadIdx.x == 0) {
+    sh.team.top = a.G.L.top;
+    sh.team.ops = 0;
+    sh.team.fail = sh.team.wrong = 0;
+    sh.stop = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    help(a, &sh, reinterpret_cast<uint2 *>(heap_top + ((sizeof(float) + sizeof(uint2)) << levels)), edit_runs(levels));
+    return;
+  }
+  Simp s(a, heap_top, levels, &sh);
   s.run();
-  a.stats[3] = s.A.G.ops;
-  if (s.A.G.fail) a.stats[4] |= ST_SIMPLIFY_LIMIT;
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    a.stats[3] = s.W.G.ops;
+    if (s.W.G.fail) a.stats[4] |= ST_SIMPLIFY_LIMIT;
+    s.W.G.L.top = sh.team.top;
+    args[blockIdx.x].G = s.W.G;  // for k_unsimplify
+    args[blockIdx.x].ncanc = s.ncanc;
+    args[blockIdx.x].loose = s.loose;
+    sh.stop = 1;
+  }
+  __syncwarp();
+  bar_arrive(BAR_GO);
+}
+
+// un_simplify (grid_mscomplex.cpp:514-526): the cancelled pairs are
+// uncancelled in reverse order, one complex per block.  A pair's
+// uncancellation rewrites one asc and one des list of its own points, the asc
+// list from asc lists of earlier pairs' points that no later pair changes,
+// the des list from their des lists.  So the block's warps take the lists in
+// order, and a warp waits only for the lists that its own one names (`ord`,
+// `done`): a list is a chain of ~10 dependent memory round trips (3,200 cycles
+// on one warp), and up to 16 of them overlap (2,775 pairs of a 2047x1365 field:
+// 7.6 ms on one warp, 3.5 ms here).  They are taken in order, so the
+// first one not yet done never waits.  A cancellation list with a pair that
+// was not connected (its points may be on the list twice) goes through one
+// warp in plain order.
+constexpr uint32_t DONE_WORDS = 4096;  // lists tracked in shared memory, 32 a word; more: in the resubmit list's memory
+__global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, uint32_t stage_runs, uint32_t shared_runs) {
+  extern __shared__ __align__(16) unsigned char un_smem[];
+  __shared__ TeamState team;
+  if (blockIdx.x >= (unsigned)n) return;
+  const SimpArgs a = args[blockIdx.x];
+  if (a.G.fail || a.stats[4] != 0 || a.ncanc == 0) return;  // (block-uniform)
+  WarpGraph W;
+  W.G = a.G;
+  W.lane = threadIdx.x & 31;
+  uint2 *buf = reinterpret_cast<uint2 *>(un_smem);
+  W.stage = buf + (size_t)(threadIdx.x >> 5) * stage_runs;
+  W.nstage = stage_runs;
+  W.shared_stage = buf + (size_t)(blockDim.x >> 5) * stage_runs;
+  W.nshared_stage = shared_runs;
+  W.team = &team;
+  const uint32_t words = (2 * a.ncanc + 31) / 32;
+  W.done = words <= DONE_WORDS ? reinterpret_cast<uint32_t *>(W.shared_stage + shared_runs) : reinterpret_cast<uint32_t *>(a.resub);
+  if (threadIdx.x == 0) {
+    team.top = a.G.L.top;
+    team.ops = a.G.ops;
+    team.ticket = 2ull * a.ncanc;
+    team.fail = team.wrong = 0;
+    team.lock = 0;
+  }
+  for (uint32_t i = threadIdx.x; i < a.G.ncp; i += blockDim.x) a.meta[i] = 0;
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) W.done[i] = 0;
+  __syncthreads();
+  if (!a.loose) {
+    for (uint32_t k = threadIdx.x; k < a.ncanc; k += blockDim.x) {
+      const uint2 c = a.canc[k];
+      a.meta[c.x] = a.meta[c.y] = k + 1;  // (a point is cancelled once)
+    }
+    __syncthreads();
+    W.ord = a.meta;
+    for (;;) {
+      unsigned long long t = 0;
+      if (W.lane == 0) t = atomicAdd(&team.ticket, ~0ull);  // takes one: from the last pair on, asc before des
+      t = __shfl_sync(FULL_WARP, t, 0);
+      if (t == 0 || t > 2ull * a.ncanc) break;  // none left
+      if (__any_sync(FULL_WARP, *(volatile uint32_t *)&team.fail || *(volatile uint32_t *)&team.wrong)) break;
+      const uint32_t k = (uint32_t)((t - 1) / 2), i = (uint32_t)(t & 1);
+      const uint2 c = a.canc[k];
+      if (!W.uncancel_list(c.x, c.y, (int)i, k + 1)) team.wrong = 1;
+      if (W.G.fail) {
+        team.fail = 1;
+        break;
+      }
+      __threadfence_block();
+      __syncwarp();
+      if (W.lane == 0) atomicOr(&W.done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < a.ncanc; k += blockDim.x) {
+      const uint2 c = a.canc[k];
+      a.G.flags[c.x] &= ~F_CANCELLED;
+      a.G.flags[c.y] &= ~F_CANCELLED;
+    }
+  } else if (threadIdx.x < 32) {
+    for (uint32_t k = a.ncanc; k-- > 0 && !team.fail && !team.wrong;) {
+      const uint2 c = a.canc[k];
+      if (!W.uncancel_pairs(c.x, c.y)) team.wrong = 1;
+      if (W.G.fail) team.fail = 1;
+      __syncwarp();
+    }
+  }
+  if (W.lane == 0) atomicAdd(&team.ops, W.G.ops - a.G.ops);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.stats[3] = team.ops;
+    if (team.wrong) a.stats[4] |= ST_INVARIANT;  // (the other warps stopped for it)
+    else if (team.fail || team.ops > a.G.max_ops) a.stats[4] |= ST_SIMPLIFY_LIMIT;
+  }
+}
+
+static cudaError_t launch_simplify(SimpArgs *args, int n, int levels, cudaStream_t st) {
+  // warps and runs of scratch per block: one block per SM, or several when a batch has more complexes than SMs
+  const int warps = n <= 152 ? 16 : 8;
+  const uint32_t own = n <= 152 ? 1024 : 512, shared = n <= 152 ? 8192 : 4096;
+  constexpr size_t un_max = sizeof(uint2) * (16 * 1024 + 8192) + sizeof(uint32_t) * DONE_WORDS;
+  static const cudaError_t attr = [] {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_simplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)top_bytes(TOP_LEVELS));
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_unsimplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)un_max);
+  }();
+  if (attr != cudaSuccess) return attr;
+  k_simplify<<<n, 32 * SIMP_WARPS, top_bytes(levels), st>>>(args, n, levels);
+  k_unsimplify<<<n, 32 * warps, sizeof(uint2) * (warps * own + shared) + sizeof(uint32_t) * DONE_WORDS, st>>>(args, n, own, shared);
+  DMSC_LAUNCHED(2);
+  return cudaGetLastError();
 }
 
 // CSR (expanded, ascending) -> run-length lists.  Capacity of a list is its
@@ -485,14 +840,15 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
   unsigned long long des_base = (unsigned long long)io.nasc + 4ull * ncp;
   unsigned long long base_top = des_base + (unsigned long long)io.ndes + 4ull * ncp;
   unsigned long long pool_cap = base_top + (io.pool_extra ? io.pool_extra : (2 * base_top + (1ull << 22)));
-  unsigned long long heap_cap = io.heap_cap ? io.heap_cap : (4ull * io.ndes + (1ull << 20));
-  unsigned long long tmp_cap = io.tmp_cap ? io.tmp_cap : (1ull << 22);
+  const unsigned long long heap_cap = std::min(io.heap_cap ? io.heap_cap : (4ull * io.ndes + (1ull << 20)), HEAP_MAX);
+  // scratch runs: two per added value of a merged list (edit_list), per helper warp
+  unsigned long long tmp_cap = io.tmp_cap ? io.tmp_cap : std::max(1ull << 22, 2ull * HELPERS * ncp);
   if (pool_cap > 0xffffffffull) return cudaErrorInvalidValue;  // list offsets are 32-bit
   if (ncp > IDX_MASK) return cudaErrorInvalidValue;               // heap entries hold 29-bit indices
   auto rnd = [](size_t n) { return (n + 255) / 256 * 256; };
   size_t sizes[] = {sizeof(uint32_t) * 2 * ncp, sizeof(uint32_t) * 2 * ncp, sizeof(uint32_t) * 2 * ncp,
-                    sizeof(uint32_t) * 2 * ncp, sizeof(uint2) * pool_cap, sizeof(uint2) * tmp_cap, sizeof(HeapEnt) * heap_cap,
-                    sizeof(HeapEnt) * heap_cap, sizeof(uint2) * (ncp + 1), sizeof(unsigned long long) * 8,
+                    sizeof(uint32_t) * 2 * ncp, sizeof(uint2) * pool_cap, sizeof(uint2) * tmp_cap, sizeof(float) * (heap_cap + 2),
+                    sizeof(uint2) * (heap_cap + 2), sizeof(HeapEnt) * heap_cap, sizeof(uint2) * (ncp + 1), sizeof(unsigned long long) * 8,
                     sizeof(uint8_t) * (ncp + 1), sizeof(uint32_t) * (ncp + 1), sizeof(uint32_t) * (ncp + 1),
                     sizeof(HeapEnt) * ((size_t)io.ndes + 1), sizeof(SimpArgs), sizeof(uint32_t) * (ncp + 1)};
   size_t bytes = 0;
@@ -518,7 +874,8 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
   G.L.pool_cap = pool_cap;
   G.tmp = (uint2 *)take();
   G.tmp_cap = tmp_cap;
-  a.heap = (HeapEnt *)take();
+  a.hkey = (float *)take();
+  a.hab = (uint2 *)take();
   a.heap_cap = heap_cap;
   a.resub = (HeapEnt *)take();
   a.canc = (uint2 *)take();
@@ -550,11 +907,8 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     k_simp_meta<<<blocks_for(ncp), 256, 0, st>>>(dargs);
     k_simp_prep<<<blocks_for(ncp), 256, 0, st>>>(dargs);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_simplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAP_TOP_BYTES);
-    if (attr != cudaSuccess) return attr;
-    k_simplify<<<1, 32, HEAP_TOP_BYTES, st>>>(a);
-    DMSC_LAUNCHED(3);
+    DMSC_LAUNCHED(2);
+    if ((e = launch_simplify(dargs, 1, TOP_LEVELS, st)) != cudaSuccess) return e;
   }
   e = cudaMemcpyAsync(io.host_stats, a.stats, sizeof(unsigned long long) * 5, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -600,18 +954,6 @@ void simplify_release(SimplifyIO &io, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // batches: one block per complex to simplify, all in one launch
 // ---------------------------------------------------------------------------
-__global__ void k_simplify_batch(SimpArgs *args, int n, unsigned ntop) {
-  extern __shared__ HeapEnt heap_top[];
-  if (threadIdx.x != 0 || blockIdx.x >= (unsigned)n) return;
-  Simp s;
-  s.A = args[blockIdx.x];
-  s.top = heap_top;
-  s.ntop = ntop;
-  s.run();
-  s.A.stats[3] = s.A.G.ops;
-  if (s.A.G.fail) s.A.stats[4] |= ST_SIMPLIFY_LIMIT;
-}
-
 struct BatchSimplifyWork {
   char *buf = nullptr;
   uint32_t *off = nullptr, *nrun = nullptr, *lcap = nullptr, *total = nullptr, *lens = nullptr;
@@ -632,17 +974,19 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
   auto grow_of = [&](unsigned long long na, unsigned long long nd, unsigned long long n) {
     return sc * (4 * (na + nd + 8 * n) + 16384);
   };
-  auto heap_of = [&](unsigned long long nd) { return sc * (8 * nd + 16384); };
-  auto tmp_of = [&](unsigned long long na, unsigned long long nd) { return sc * (4 * (na + nd) + 16384); };
+  auto heap_of = [&](unsigned long long nd) { return std::min(sc * (8 * nd + 16384), HEAP_MAX); };  // (even)
+  auto tmp_of = [&](unsigned long long na, unsigned long long nd, unsigned long long n) {
+    return sc * (4 * (na + nd) + 16384) + 2 * HELPERS * n;
+  };
   for (int g = 0; g < io.ngrids; ++g) {
     const unsigned long long n = io.cpb[g + 1] - io.cpb[g];
     if (!(io.tresh[g] > 0.0) || n == 0) continue;
     const unsigned long long na = io.abase[g + 1] - io.abase[g], nd = io.dbase[g + 1] - io.dbase[g];
     which.push_back(g);
     grow += grow_of(na, nd, n);
-    heap += heap_of(nd);
+    heap += heap_of(nd) + 2;
     canc += n + 1;
-    tmp += tmp_of(na, nd);
+    tmp += tmp_of(na, nd, n);
     init += nd + 1;
   }
   const unsigned long long pool_cap = base_top + grow;
@@ -659,7 +1003,8 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
   const int ns = (int)which.size();
   auto rnd = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t sizes[] = {4ull * 2 * ncp, 4ull * 2 * ncp, 4ull * 2 * ncp, 4ull * 2 * ncp, 4ull * (ncp + 1),
-                          sizeof(uint2) * pool_cap, sizeof(uint2) * tmp, sizeof(HeapEnt) * heap, sizeof(HeapEnt) * heap,
+                          sizeof(uint2) * pool_cap, sizeof(uint2) * tmp, sizeof(float) * heap, sizeof(uint2) * heap,
+                          sizeof(HeapEnt) * heap,
                           sizeof(uint2) * canc, sizeof(unsigned long long) * 8 * (size_t)(ns + 1),
                           sizeof(SimpArgs) * (size_t)(ns + 1), sizeof(HeapEnt) * (init + 1), 4ull * (ncp + 1)};
   size_t bytes = 0;
@@ -675,7 +1020,8 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
   w->lens = (uint32_t *)take();
   w->pool = (uint2 *)take();
   uint2 *dtmp = (uint2 *)take();
-  HeapEnt *dheap = (HeapEnt *)take();
+  float *dhkey = (float *)take();
+  uint2 *dhab = (uint2 *)take();
   HeapEnt *dres = (HeapEnt *)take();
   uint2 *dcanc = (uint2 *)take();
   w->dstats = (unsigned long long *)take();
@@ -708,17 +1054,18 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
     top += grow_of(na, nd, n);
     G.L.pool_cap = top;
     G.tmp = dtmp + to;
-    G.tmp_cap = tmp_of(na, nd);
+    G.tmp_cap = tmp_of(na, nd, n);
     to += G.tmp_cap;
     G.max_ops = io.max_ops;
     G.ops = 0;
     G.fail = false;
     a.fn = io.fn + c0;
     a.meta = dmeta + c0;
-    a.heap = dheap + ho;
+    a.hkey = dhkey + ho;
+    a.hab = dhab + ho;
     a.resub = dres + ho;
     a.heap_cap = heap_of(nd);
-    ho += a.heap_cap;
+    ho += a.heap_cap + 2;
     a.canc = dcanc + co;
     co += n + 1;
     a.aoff = io.aoff + c0; a.asc = io.asc; a.doff = io.doff + c0; a.des = io.des;
@@ -731,18 +1078,14 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
   }
   if (e == cudaSuccess && ns) e = cudaMemcpyAsync(w->dargs, args.data(), sizeof(SimpArgs) * ns, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && ns) {
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_simplify_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAP_TOP_BYTES);
-    if (attr != cudaSuccess) return attr;
     // one grid per SM can keep 14 heap levels in shared memory; more grids
     // than SMs keep 13, two per SM (measured on the 1000-grid workload: 13
     // levels 108.8 ms, 12 levels (four per SM) 113.8, 14 levels 122.4)
-    const unsigned ntop = ns <= 152 ? (unsigned)HEAP_TOP : (1u << 13) - 1;
+    const int levels = ns <= 152 ? TOP_LEVELS : TOP_LEVELS_BATCH;
     k_simp_meta<<<dim3(64, (unsigned)ns), 256, 0, st>>>(w->dargs);
     k_simp_prep<<<dim3(64, (unsigned)ns), 256, 0, st>>>(w->dargs);
-    k_simplify_batch<<<ns, 32, sizeof(HeapEnt) * ntop, st>>>(w->dargs, ns, ntop);
-    DMSC_LAUNCHED(3);
-    e = cudaGetLastError();
+    DMSC_LAUNCHED(2);
+    e = launch_simplify(w->dargs, ns, levels, st);
   }
   std::vector<unsigned long long> hs(8 * (size_t)(ns + 1), 0);
   if (e == cudaSuccess && ns) e = cudaMemcpyAsync(hs.data(), w->dstats, sizeof(unsigned long long) * 8 * ns, cudaMemcpyDeviceToHost, st);
