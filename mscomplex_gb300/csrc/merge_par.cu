@@ -17,12 +17,11 @@
 //     uncancelled points -- counts, a scan, a scatter, and a sort of each list
 //     by index (the ascending order in which a std::multiset iterates);
 //   * the cancellations along the shared boundary (:124-153), row-major and
-//     order dependent: one thread per merge, on the mutable graph
-//     (merge_up_cancel in merge_graph.cuh), all merges of the level in one
-//     launch.
+//     order dependent: one block per merge, on the mutable graph
+//     (k_merge_up_seq), all merges of the level in one launch.
 // merge_down (:158-322) splits into
-//   * the uncancellations along the shared boundary (:172-201): one thread
-//     per parent (merge_down_boundary), all merges of the level in one launch;
+//   * the uncancellations along the shared boundary (:172-201): one block per
+//     parent (k_merge_down_seq), all merges of the level in one launch;
 //   * the parent's boundary-cancelable points pushed into each child
 //     (:207-281): the points it adds to the child are numbered by a scan over
 //     the sequence of additions the reference's loop makes (down_child);
@@ -45,6 +44,7 @@
 #include "grid_types.h"
 #include "host_pool.h"
 #include "merge_graph.cuh"
+#include "warp_graph.cuh"
 
 namespace dmsc {
 
@@ -565,7 +565,7 @@ __global__ void k_dc_write(DcArgs a, uint32_t n, const uint32_t *src) {
 }
 
 // ---------------------------------------------------------------------------
-// the one-thread steps of a level, one block per job
+// the boundary steps of a level, one block per job
 // ---------------------------------------------------------------------------
 enum SeqKind : int { SEQ_UP_CANCEL = 0, SEQ_DOWN_BOUNDARY = 1 };
 struct SeqJob {
@@ -613,18 +613,300 @@ __global__ void k_seq_prefetch(const MGraph *graphs, const SeqJob *jobs, uint32_
   if (acc == 0x9E3779B9u && sink) *sink = acc;
 }
 
-// The graphs are worked on as local copies of their descriptors: the
-// pointers and counters stay in registers instead of being reloaded from
-// global memory after every store through a list pointer.
-__global__ void k_merge_seq(MGraph *graphs, const SeqJob *jobs, int njobs, uint32_t *status) {
+// merge_up's boundary cancellations, one job per block.  The first warp walks
+// the boundary cells in the loop's order, 32 at a time: their lanes look the
+// cells up side by side (cell -> point -> flags and pair -> the pair's cell)
+// and drop those the loop would skip whatever happens before their turn; then
+// the cells left are done one after the other (warp_graph.cuh).  A
+// cancellation's list edits are shared by SEQ_WARPS warps: the short lists are
+// the first warp's, the longer ones go round.  A cancellation is a chain of
+// memory round trips (one thread took 19,000 cycles for one on 2048^2 white
+// noise; here 5,000), so one more warp runs a batch of cells ahead and brings what
+// they will read into L1: their points, both points' lists, the neighbours' list
+// descriptors and lists.
+constexpr int SEQ_WARPS = 4;
+constexpr uint32_t SEQ_STAGE = 512;  // runs of scratch per warp in shared memory
+struct SeqShared {
+  TeamState team;
+  WarpGraph::Pair pair;
+  int stop;
+  long long at;  // first cell of the batch the first warp is at
+  uint2 stage[SEQ_WARPS * SEQ_STAGE];
+};
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// Into L1: point c's lists, and the flags, list descriptors and first list
+// line of their first neighbours.
+__device__ __forceinline__ void warm_point(const MGraph &M, uint32_t c) {
+  const uint2 off = reinterpret_cast<const uint2 *>(M.G.L.off)[c], n = reinterpret_cast<const uint2 *>(M.G.L.nrun)[c];
+  prefetch_l1(M.G.L.total + 2 * c);
+  constexpr uint32_t Q = 12;
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    const uint2 *r = M.G.L.pool + (w ? off.y : off.x);
+    const uint32_t m = w ? n.y : n.x;
+    uint32_t v[Q], o[Q];
+#pragma unroll
+    for (uint32_t q = 0; q < Q; ++q) v[q] = q < m ? r[q].x : M.G.ncp;
+#pragma unroll
+    for (uint32_t q = 0; q < Q; ++q) {
+      o[q] = 0;
+      if (v[q] < M.G.ncp) {
+        o[q] = M.G.L.off[2 * v[q] + 1 - w];
+        prefetch_l1(M.G.flags + v[q]);
+        prefetch_l1(M.G.L.nrun + 2 * v[q]);
+        prefetch_l1(M.G.L.cap + 2 * v[q]);
+        prefetch_l1(M.G.L.total + 2 * v[q]);
+      }
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < Q; ++q)
+      if (v[q] < M.G.ncp) prefetch_l1(M.G.L.pool + o[q]);
+  }
+}
+
+// Whether the loop would act on the point si of cell (x, y) with partner pi.
+__device__ __forceinline__ bool cell_acts(const MGraph &M, int x, int y, uint32_t pi) {
+  const uint32_t p = M.G.cellid[pi];
+  return (M.rect.interior(x, y) || M.ext.boundary(x, y)) && (M.rect.interior(px_(p), py_(p)) || M.ext.boundary(px_(p), py_(p)));
+}
+
+// Cell t of the boundary, for merge_up: its point si and partner pi; 1 where
+// the loop may act at its turn, 0 where it passes, 2 no point there, 3 a
+// partner outside the complex.  (A cell already cancelled, or not
+// boundary-cancelable, stays so.)
+__device__ __forceinline__ int up_cell(const MGraph &M, const CRect &ixn, long long w, long long t, uint32_t &si, uint32_t &pi) {
+  const int x = ixn.l + (int)(t % w), y = ixn.b + (int)(t / w);
+  si = M.find(pack_cellid(x, y));
+  if (si >= M.G.ncp) return 2;
+  const uint8_t f = M.G.flags[si];
+  pi = M.G.pair_idx[si];
+  if (!(f & F_BCANCEL) || (f & F_CANCELLED)) return 0;
+  return pi >= M.G.ncp ? 3 : cell_acts(M, x, y, pi) ? 1 : 0;
+}
+__device__ __forceinline__ void seq_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * SEQ_WARPS) : "memory"); }
+
+__global__ void __launch_bounds__(32 * (SEQ_WARPS + 1)) k_merge_up_seq(MGraph *graphs, const SeqJob *jobs, int njobs, uint32_t *status) {
+  __shared__ SeqShared sh;
   const int b = blockIdx.x;
-  if (b >= njobs || threadIdx.x != 0) return;
+  if (b >= njobs) return;
   const SeqJob jb = jobs[b];
-  MGraph g0 = graphs[jb.g0];
-  if (jb.kind == SEQ_UP_CANCEL) merge_up_cancel(g0, jb.ixn, status);
-  else merge_down_boundary(g0, jb.ixn, status);
-  if (g0.G.fail) set_status(status, ST_SIMPLIFY_LIMIT);
-  graphs[jb.g0] = g0;
+  const MGraph M = graphs[jb.g0];  // (a copy of the descriptor: pointers stay in registers)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long w = jb.ixn.r - jb.ixn.l + 1, n = w * (jb.ixn.t - jb.ixn.b + 1);
+  if (threadIdx.x == 0) {
+    sh.team.top = M.G.L.top;
+    sh.team.fail = 0;
+    sh.stop = 0;
+    sh.at = 0;
+  }
+  __syncthreads();
+  if (warp == SEQ_WARPS) {  // reads ahead: at most one batch beyond the first warp's
+    for (long long t0 = 0; t0 < n; t0 += 32) {
+      for (long long polls = 0; *(volatile long long *)&sh.at + 32 < t0 && !*(volatile int *)&sh.stop && polls < (1ll << 26); ++polls) __nanosleep(200);
+      if (*(volatile int *)&sh.stop) break;
+      uint32_t si = 0, pi = 0;
+      if (t0 + lane < n && up_cell(M, jb.ixn, w, t0 + lane, si, pi) == 1) {
+        warm_point(M, si);
+        warm_point(M, pi);
+      }
+      __syncwarp();
+    }
+    return;
+  }
+  WarpGraph W;
+  W.G = M.G;
+  W.lane = lane;
+  W.team = &sh.team;
+  W.stage = sh.stage + warp * SEQ_STAGE;
+  W.nstage = SEQ_STAGE;
+  W.G.tmp_cap = M.G.tmp_cap / SEQ_WARPS;
+  W.G.tmp = M.G.tmp + warp * W.G.tmp_cap;
+  if (warp > 0) {
+    for (;;) {
+      seq_barrier();
+      if (sh.stop) return;
+      W.edit_neighbours(sh.pair, warp, SEQ_WARPS);
+      if (W.G.fail) sh.team.fail = 1;
+      seq_barrier();
+    }
+  }
+  bool stop = false;
+  for (long long t0 = 0; t0 < n && !stop; t0 += 32) {
+    if (lane == 0) *(volatile long long *)&sh.at = t0;
+    uint32_t si = 0, pi = 0;
+    const int todo = t0 + lane < n ? up_cell(M, jb.ixn, w, t0 + lane, si, pi) : 0;
+    __syncwarp();
+    for (unsigned left = __ballot_sync(FULL_WARP, todo != 0); left && !stop; left &= left - 1) {
+      const int s = __ffs(left) - 1;
+      const int what = __shfl_sync(FULL_WARP, todo, s);
+      const uint32_t c = __shfl_sync(FULL_WARP, si, s), d = __shfl_sync(FULL_WARP, pi, s);
+      if (what != 2 && (M.G.flags[c] & F_CANCELLED)) continue;  // with an earlier cell
+      if (what != 1) {  // "missing common bndry cp", or a partner outside the complex
+        if (lane == 0) set_status(status, ST_INVARIANT);
+        stop = true;
+        break;
+      }
+      WarpGraph::Pair q{reinterpret_cast<const uint2 *>(M.G.L.off)[c], reinterpret_cast<const uint2 *>(M.G.L.off)[d],
+                        reinterpret_cast<const uint2 *>(M.G.L.nrun)[c], reinterpret_cast<const uint2 *>(M.G.L.nrun)[d], c, d};
+      if (!W.orient(q)) continue;
+      if (lane == 0) sh.pair = q;
+      seq_barrier();
+      W.edit_neighbours(q, 0, SEQ_WARPS);
+      if (W.G.fail) sh.team.fail = 1;
+      seq_barrier();
+      W.close(q, 0);
+      __syncwarp();
+      if (sh.team.fail) stop = true;
+    }
+  }
+  if (lane == 0) {
+    *(volatile int *)&sh.stop = 1;
+    MGraph g = M;
+    g.G.fail = sh.team.fail != 0;
+    g.G.ops = W.G.ops;
+    g.G.L.top = sh.team.top;
+    if (g.G.fail) set_status(status, ST_SIMPLIFY_LIMIT);
+    graphs[jb.g0] = g;
+  }
+  __syncwarp();
+  seq_barrier();
+}
+
+// merge_down's boundary uncancellations, one job per block.  The loop runs in
+// reverse row-major order over the cells whose point is cancelled; a pair's
+// two lists are rewritten from lists of pairs uncancelled before it, so the
+// block's warps take them in the loop's order and wait only for the lists
+// their own name (WarpGraph::uncancel_shared).  Before that the whole block
+// lists the pairs: a pair with both points on the boundary belongs to the cell
+// the loop meets first.  A pair whose points do not name each other takes the
+// job to the plain order on one warp.  (2048^2 white noise in 16 pieces, all
+// levels: 19.5 ms on one thread, 1.6 ms here.)
+constexpr int DOWN_WARPS = 16;
+constexpr uint32_t DOWN_STAGE = 512, DOWN_SHARED = 4096;  // runs of scratch: each warp's own, the one they share
+struct DownWork {
+  uint32_t *ord;  // per point of the job's graph (zeroed)
+  uint2 *pairs;   // room for the boundary's cells
+};
+constexpr int DOWN_CELLS = 32768;  // cell coordinates are below 2^15, and a boundary is one cell wide
+constexpr uint32_t DOWN_DONE = 2 * DOWN_CELLS / 32;  // words
+constexpr size_t DOWN_SMEM = sizeof(uint2) * (DOWN_WARPS * DOWN_STAGE + DOWN_SHARED) + sizeof(uint32_t) * DOWN_DONE;
+__global__ void __launch_bounds__(32 * DOWN_WARPS, 1) k_merge_down_seq(MGraph *graphs, const SeqJob *jobs, int njobs,
+                                                                       const DownWork *works, uint32_t *status) {
+  extern __shared__ __align__(16) unsigned char down_smem[];
+  __shared__ TeamState team;
+  __shared__ uint32_t count[DOWN_WARPS];
+  __shared__ int odd;
+  const int b = blockIdx.x;
+  if (b >= njobs) return;
+  const SeqJob jb = jobs[b];
+  const MGraph M = graphs[jb.g0];
+  const DownWork wk = works[b];
+  const int warp = threadIdx.x >> 5;
+  WarpGraph W;
+  W.G = M.G;
+  W.lane = threadIdx.x & 31;
+  W.team = &team;
+  uint2 *buf = reinterpret_cast<uint2 *>(down_smem);
+  W.stage = buf + (size_t)warp * DOWN_STAGE;
+  W.nstage = DOWN_STAGE;
+  W.shared_stage = buf + DOWN_WARPS * DOWN_STAGE;
+  W.nshared_stage = DOWN_SHARED;
+  W.done = reinterpret_cast<uint32_t *>(W.shared_stage + DOWN_SHARED);
+  for (uint32_t i = threadIdx.x; i < DOWN_DONE; i += blockDim.x) W.done[i] = 0;
+  const long long w = jb.ixn.r - jb.ixn.l + 1, n = w * (jb.ixn.t - jb.ixn.b + 1);
+  if (threadIdx.x == 0) {
+    team.top = M.G.L.top;
+    team.fail = team.wrong = 0;
+    team.lock = 0;
+    odd = n > DOWN_CELLS;
+  }
+  __syncthreads();
+  // cell t's point si and its partner pi: 1 where the loop acts on them, 0
+  // where it passes, 2 no point there, 3 a partner outside the complex
+  auto cell = [&](long long t, uint32_t &si, uint32_t &pi) -> int {
+    const int x = jb.ixn.l + (int)(t % w), y = jb.ixn.b + (int)(t / w);
+    si = M.find(pack_cellid(x, y));
+    if (si >= M.G.ncp) return 2;
+    if (!(M.G.flags[si] & F_CANCELLED)) return 0;
+    pi = M.G.pair_idx[si];
+    return pi >= M.G.ncp ? 3 : cell_acts(M, x, y, pi) ? 1 : 0;
+  };
+  uint32_t si = 0, pi = 0;
+  for (long long t = threadIdx.x; t < n; t += blockDim.x) {
+    const int what = cell(t, si, pi);
+    if (what == 1) {
+      atomicMax(&wk.ord[si], (uint32_t)t + 1);
+      atomicMax(&wk.ord[pi], (uint32_t)t + 1);
+      if (M.G.pair_idx[pi] != si) odd = 1;
+    }
+    if (what == 2) team.wrong = 1;  // "missing common bndry cp"
+    if (what == 3) odd = 1;
+  }
+  __syncthreads();
+  if (!team.wrong && !odd) {
+    // the pairs in cell order: each warp its part of the boundary
+    const long long part = ((n + DOWN_WARPS - 1) / DOWN_WARPS + 31) / 32 * 32, c0 = part * warp, c1 = min(c0 + part, n);
+    uint32_t mine = 0;
+    for (long long t0 = c0; t0 < c1; t0 += 32) {
+      const long long t = t0 + W.lane;
+      const bool own = t < c1 && cell(t, si, pi) == 1 && wk.ord[si] == (uint32_t)t + 1;
+      mine += __popc(__ballot_sync(FULL_WARP, own));
+    }
+    if (W.lane == 0) count[warp] = mine;
+    __syncthreads();
+    uint32_t at = 0, np = 0;
+    for (int k = 0; k < DOWN_WARPS; ++k) {
+      if (k < warp) at += count[k];
+      np += count[k];
+    }
+    for (long long t0 = c0; t0 < c1; t0 += 32) {
+      const long long t = t0 + W.lane;
+      const bool own = t < c1 && cell(t, si, pi) == 1 && wk.ord[si] == (uint32_t)t + 1;
+      const unsigned m = __ballot_sync(FULL_WARP, own);
+      if (own) {
+        const uint2 *p = M.G.runs(2 * si);
+        uint32_t lo = 0, hi = M.G.L.nrun[2 * si];
+        while (lo < hi) {
+          const uint32_t c = (lo + hi) >> 1;
+          if (p[c].x < pi) lo = c + 1; else hi = c;
+        }
+        const bool first = lo < M.G.L.nrun[2 * si] && p[lo].x == pi;  // asc(si) holds pi
+        wk.pairs[at + __popc(m & W.lt())] = first ? make_uint2(si, pi) : make_uint2(pi, si);
+      }
+      at += __popc(m);
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < np; k += blockDim.x) {
+      const uint2 c = wk.pairs[k];
+      wk.ord[c.x] = wk.ord[c.y] = k + 1;
+    }
+    if (threadIdx.x == 0) team.ticket = 2ull * np;
+    __syncthreads();
+    W.ord = wk.ord;
+    W.uncancel_shared(wk.pairs, np);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < np; k += blockDim.x) {
+      const uint2 c = wk.pairs[k];
+      M.G.flags[c.x] &= ~F_CANCELLED;
+      M.G.flags[c.y] &= ~F_CANCELLED;
+    }
+  } else if (!team.wrong && warp == 0) {
+    for (long long t = n - 1; t >= 0 && !team.wrong && !W.G.fail; --t) {
+      const int what = cell(t, si, pi);
+      if (what >= 2 || (what == 1 && !W.uncancel_pairs(si, pi))) team.wrong = 1;
+      if (W.G.fail) team.fail = 1;
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    MGraph g = M;
+    g.G.fail = team.fail != 0 && !team.wrong;
+    g.G.L.top = team.top;
+    if (team.wrong) set_status(status, ST_INVARIANT);  // (the other warps stopped for it)
+    else if (team.fail) set_status(status, ST_SIMPLIFY_LIMIT);
+    graphs[jb.g0] = g;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -733,7 +1015,7 @@ __global__ void __launch_bounds__(ROUND_THREADS, 1) k_merge_up_rounds(MGraph *gr
   MGraph g = graphs[jb.g0];  // every thread's own descriptor copy, read before any write-back
   const long long w = jb.ixn.r - jb.ixn.l + 1, h = jb.ixn.t - jb.ixn.b + 1, n = w * h;
   unsigned long long *slot = slots[b];
-  if (n > ROUND_TASKS || !slot || jb.win <= 0) {  // one thread, as k_merge_seq
+  if (n > ROUND_TASKS || !slot || jb.win <= 0) {  // one thread
     if (threadIdx.x == 0) {
       merge_up_cancel(g, jb.ixn, status);
       if (g.G.fail) set_status(status, ST_SIMPLIFY_LIMIT);
@@ -839,7 +1121,7 @@ __global__ void __launch_bounds__(ROUND_THREADS, 1) k_merge_up_rounds(MGraph *gr
 
 MGraph &mg(MGraphHost &h) { return *reinterpret_cast<MGraph *>(h.raw); }
 
-// List pool (runs) beyond the lists themselves for the one-thread steps
+// List pool (runs) beyond the lists themselves for the steps
 // along a shared boundary: lists there relocate to the pool top as they
 // grow (the graphs start without slack); retries multiply it.
 unsigned long long boundary_room(const int ixn[4]) {
@@ -866,17 +1148,24 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
   char *buf = nullptr;
   const size_t nj = jobs.size();
   const size_t gb = sizeof(MGraph) * ng, jbytes = sizeof(SeqJob) * nj;
-  // merge_up's jobs run in rounds: per job a slot per critical point of its
-  // graph (round-tagged keys, all ones = empty) and a pool top
-  const bool rounds = jobs[0].kind == SEQ_UP_CANCEL;
-  std::vector<size_t> soff(nj, 0);
+  // merge_up's jobs in rounds (a window set): per job a slot per critical point
+  // of its graph (round-tagged keys, all ones = empty).  merge_down: per job an
+  // order word per critical point (zero), then the boundary's pairs.
+  const bool down = jobs[0].kind == SEQ_DOWN_BOUNDARY, rounds = !down && jobs[0].win > 0;
+  std::vector<size_t> soff(nj, 0), poff(nj, 0);
   size_t sbytes = 0;
-  if (rounds)
-    for (size_t k = 0; k < nj; ++k) {
-      soff[k] = sbytes;
-      sbytes += 8ull * ((mg(*graphs[jobs[k].g0]).G.ncp + 1 + 31) / 32 * 32);
-    }
-  const size_t head = (gb + 15) / 16 * 16 + (jbytes + 15) / 16 * 16, pbytes = rounds ? (8ull * nj + 15) / 16 * 16 : 0;
+  for (size_t k = 0; k < nj && (rounds || down); ++k) {
+    soff[k] = sbytes;
+    sbytes += (rounds ? 8ull : 4ull) * ((mg(*graphs[jobs[k].g0]).G.ncp + 1 + 31) / 32 * 32);
+  }
+  const size_t obytes = sbytes;
+  for (size_t k = 0; k < nj && down; ++k) {
+    const CRect &x = jobs[k].ixn;
+    poff[k] = sbytes;
+    sbytes += sizeof(uint2) * ((size_t)(x.r - x.l + 1) * (x.t - x.b + 1) + 15) / 16 * 16;
+  }
+  const size_t head = (gb + 15) / 16 * 16 + (jbytes + 15) / 16 * 16;
+  const size_t pbytes = ((rounds ? 8ull : down ? sizeof(DownWork) : 0ull) * nj + 15) / 16 * 16;
   cudaError_t e = cudaMallocAsync((void **)&buf, head + pbytes + sbytes + 64, st);
   if (e != cudaSuccess) return e;
   MGraph *dg = (MGraph *)buf;
@@ -894,6 +1183,14 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
     if (e == cudaSuccess) e = cudaMemsetAsync(slots, 0xFF, sbytes, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // hp is read before it goes out of scope
   }
+  if (e == cudaSuccess && down) {
+    char *base = buf + head + pbytes;
+    std::vector<DownWork> hw(nj);
+    for (size_t k = 0; k < nj; ++k) hw[k] = DownWork{(uint32_t *)(base + soff[k]), (uint2 *)(base + poff[k])};
+    e = cudaMemcpyAsync(buf + head, hw.data(), sizeof(DownWork) * nj, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, obytes, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // hw is read before it goes out of scope
+  }
   if (e == cudaSuccess) {
     k_seq_prefetch<<<dim3(64, (unsigned)nj), 256, 0, st>>>(dg, dj, nullptr);
     if (rounds) {
@@ -902,8 +1199,14 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
       e = attr;
       if (e == cudaSuccess)
         k_merge_up_rounds<<<(unsigned)nj, ROUND_THREADS, sizeof(RoundSmem), st>>>(dg, dj, (int)nj, dslot, status);
+    } else if (down) {
+      static const cudaError_t attr =
+          cudaFuncSetAttribute(k_merge_down_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DOWN_SMEM);
+      e = attr;
+      if (e == cudaSuccess)
+        k_merge_down_seq<<<(unsigned)nj, 32 * DOWN_WARPS, DOWN_SMEM, st>>>(dg, dj, (int)nj, (const DownWork *)(buf + head), status);
     } else {
-      k_merge_seq<<<(unsigned)nj, 32, 0, st>>>(dg, dj, (int)nj, status);
+      k_merge_up_seq<<<(unsigned)nj, 32 * (SEQ_WARPS + 1), 0, st>>>(dg, dj, (int)nj, status);
     }
     DMSC_LAUNCHED(2);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -1179,7 +1482,7 @@ int current_device() {
 }  // namespace
 
 // The merges of a level run side by side on their own streams (several host
-// threads); the one-thread steps of all of them run in one launch on `st`.
+// threads); the boundary steps of all of them run in one launch on `st`.
 cudaError_t merge_up_level_par(const std::vector<MergeJob> &jobs, unsigned long long grow, uint32_t *status,
                                uint32_t *stw, cudaStream_t st, double *seq_ms, long long round_window,
                                long long round_min_commits) {
@@ -1202,7 +1505,7 @@ cudaError_t merge_up_level_par(const std::vector<MergeJob> &jobs, unsigned long 
     cudaStreamSynchronize(st);
     return e;
   }
-  // the boundary cancellations, one thread per merge, on mutable graphs
+  // the boundary cancellations, one block per merge, on mutable graphs
   std::vector<MGraphHost *> gp;
   std::vector<SeqJob> seq;
   for (int k = 0; k < nj; ++k) {

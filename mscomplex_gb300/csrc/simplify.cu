@@ -727,23 +727,7 @@ __global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, ui
     }
     __syncthreads();
     W.ord = a.meta;
-    for (;;) {
-      unsigned long long t = 0;
-      if (W.lane == 0) t = atomicAdd(&team.ticket, ~0ull);  // takes one: from the last pair on, asc before des
-      t = __shfl_sync(FULL_WARP, t, 0);
-      if (t == 0 || t > 2ull * a.ncanc) break;  // none left
-      if (__any_sync(FULL_WARP, *(volatile uint32_t *)&team.fail || *(volatile uint32_t *)&team.wrong)) break;
-      const uint32_t k = (uint32_t)((t - 1) / 2), i = (uint32_t)(t & 1);
-      const uint2 c = a.canc[k];
-      if (!W.uncancel_list(c.x, c.y, (int)i, k + 1)) team.wrong = 1;
-      if (W.G.fail) {
-        team.fail = 1;
-        break;
-      }
-      __threadfence_block();
-      __syncwarp();
-      if (W.lane == 0) atomicOr(&W.done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
-    }
+    W.uncancel_shared(a.canc, a.ncanc);
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < a.ncanc; k += blockDim.x) {
       const uint2 c = a.canc[k];

@@ -6,7 +6,7 @@
 // handful of list edits whose cost is dependent memory round trips.  A pair's
 // edits all concern different lists (the neighbours' asc lists and des lists,
 // and a cell's lists hold cells of one dimension), so the warp makes them side
-// by side: up to 32 short lists (at most 8 runs, at most two added values) one
+// by side: up to 32 short lists (at most 8 runs, at most one added value) one
 // per lane, each read once into registers, edited there and written back; a
 // longer list by all lanes together, one merge for all added values and the
 // removed one.  Every list is left with the runs the
@@ -305,88 +305,63 @@ struct WarpGraph {
   }
 
   // One lane's share of cancel_pairs: list l of n runs (n <= N) takes the
-  // values ad[0..k) (ascending, k <= K) with counts mult * y and loses r's run.
-  template <int N, int K>
+  // value ad (k = 1) with count mult * ad.y and loses r's run.
+  template <int N>
   struct LaneEdit {
-    uint2 v[N], ad[K];
-    uint32_t apos[K], m, e;
-    bool fresh[K], bad;
+    uint2 v[N], ad;
+    uint32_t apos, m, e;
+    bool fresh, bad;
     unsigned long long total, ticks;
 
     __device__ __forceinline__ void load(const WarpGraph &W, bool on, const uint2 *p, uint32_t n, uint32_t tot,
-                                         const uint2 *add, uint32_t k, uint32_t mult, uint32_t r, bool mark_a, uint32_t self) {
-      bad = false;
-      ticks = 0;
-      total = tot;
-      m = n;
-      e = N;
+                                         uint2 add, uint32_t k, uint32_t mult, uint32_t r, bool mark_a, uint32_t self) {
 #pragma unroll
       for (int i = 0; i < N; ++i) v[i] = on && (uint32_t)i < n ? p[i] : make_uint2(0xffffffffu, 0u);
-      uint32_t before = 0;
+      const bool adds = on && k != 0;
+      const unsigned long long c = (unsigned long long)add.y * mult;
+      ad = make_uint2(add.x, (uint32_t)c);
+      apos = 0;
+      bad = adds && c > 0xffffffffull;
+      bool dup = false;
 #pragma unroll
-      for (int q = 0; q < K; ++q) {
-        ad[q] = add[q];
-        apos[q] = 0;
-        fresh[q] = false;
-        if (!on || (uint32_t)q >= k) continue;
-        const unsigned long long c = (unsigned long long)ad[q].y * mult;
-        ad[q].y = (uint32_t)c;
-        bool dup = false;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          apos[q] += v[i].x < ad[q].x;
-          if (v[i].x == ad[q].x) {
-            dup = true;
-            if (c > 0xffffffffull - v[i].y) bad = true;
-            v[i].y += (uint32_t)c;
-          }
-        }
-        if (c > 0xffffffffull) bad = true;
-        fresh[q] = !dup;
-        if (!dup) {
-          ticks += n - apos[q];
-          ++m;
-          before += ad[q].x < r;
-        }
-        total += c;
-        if (mark_a) {
-          ticks += c;
-          if (dup || c >= 2) W.mark(self, ad[q].x);
+      for (int i = 0; i < N; ++i) {
+        apos += v[i].x < ad.x;
+        if (adds && v[i].x == ad.x) {
+          dup = true;
+          if (c > 0xffffffffull - v[i].y) bad = true;
+          v[i].y += (uint32_t)c;
         }
       }
+      fresh = adds && !dup;
+      m = n + (fresh ? 1u : 0u);
+      ticks = fresh ? n - apos : 0u;
+      total = tot + (adds ? c : 0ull);
       if (total > 0xffffffffull) bad = true;
+      if (mark_a && adds) {
+        ticks += c;
+        if (dup || c >= 2) W.mark(self, ad.x);
+      }
+      e = N;
 #pragma unroll
       for (int i = 0; i < N; ++i)
         if (on && v[i].x == r) { e = i; total -= v[i].y; }
       if (e < N) {
-        ticks += m - (e + before);
+        ticks += m - (e + (fresh && ad.x < r ? 1u : 0u));
         --m;
       }
     }
     __device__ __forceinline__ void store(uint2 *p, uint32_t n) const {
 #pragma unroll
       for (int i = 0; i < N; ++i)
-        if ((uint32_t)i < n && (uint32_t)i != e) {
-          uint32_t to = i - (e < (uint32_t)i ? 1u : 0u);
-#pragma unroll
-          for (int q = 0; q < K; ++q) to += fresh[q] && ad[q].x < v[i].x;
-          p[to] = v[i];
-        }
-#pragma unroll
-      for (int q = 0; q < K; ++q)
-        if (fresh[q]) {
-          uint32_t to = apos[q] - (e < apos[q] ? 1u : 0u);
-#pragma unroll
-          for (int u = 0; u < q; ++u) to += fresh[u];
-          p[to] = ad[q];
-        }
+        if ((uint32_t)i < n && (uint32_t)i != e) p[i - (e < (uint32_t)i ? 1u : 0u) + (fresh && ad.x < v[i].x ? 1u : 0u)] = v[i];
+      if (fresh) p[apos - (e < apos ? 1u : 0u)] = ad;
     }
   };
   // All lanes: the edits of the lanes with `on`; false when the pass failed.
-  template <int N, int K>
+  template <int N>
   __device__ __forceinline__ bool lane_edits(bool on, uint32_t l, uint32_t n, uint32_t cap, uint32_t tot, uint32_t off,
-                                             const uint2 *add, uint32_t k, uint32_t mult, uint32_t r, bool mark_a) {
-    LaneEdit<N, K> E;
+                                             uint2 add, uint32_t k, uint32_t mult, uint32_t r, bool mark_a) {
+    LaneEdit<N> E;
     E.load(*this, on, G.L.pool + off, n, tot, add, k, mult, r, mark_a, l >> 1);
     uint32_t room = 0;  // for a list that outgrows its place
     if (on && E.m > cap) {
@@ -456,21 +431,17 @@ struct WarpGraph {
     const uint32_t nA = q.n0.x, nE0 = q.n0.y, nE1 = q.n1.x, nD = q.n1.y;
     const uint32_t tD = nA, tE0 = nA + nD, tE1 = tE0 + nE0, nt = tE1 + nE1;
     int turn = 0;  // the warp that takes the next longer list
-    // The added values of either side, when the list without the other point
-    // holds at most two (k: how many, 3 for more): from its first three runs.
-    uint2 addA[2], addD[2], fA[3], fD[3];
+    // The added value of either side where there is at most one (k: how many, 2
+    // for more): the list without the other point, from its first two runs.
+    uint2 fA[2], fD[2];
 #pragma unroll
-    for (uint32_t q = 0; q < 3; ++q) {
+    for (uint32_t q = 0; q < 2; ++q) {
       fA[q] = q < nA ? pA[q] : make_uint2(cp1, 0);
       fD[q] = q < nD ? pD[q] : make_uint2(cp0, 0);
     }
-    auto few = [](const uint2 f[3], uint32_t n, uint32_t skip, uint2 out[2]) -> uint32_t {
-      const bool s0 = f[0].x != skip, s1 = f[1].x != skip, s2 = f[2].x != skip;
-      out[0] = s0 ? f[0] : s1 ? f[1] : f[2];
-      out[1] = s0 && s1 ? f[1] : f[2];
-      return n > 3 ? 3u : (s0 ? 1u : 0u) + (s1 ? 1u : 0u) + (s2 ? 1u : 0u);
-    };
-    const uint32_t kA = few(fA, nA, cp1, addA), kD = few(fD, nD, cp0, addD);
+    const bool a0 = fA[0].x != cp1, a1 = fA[1].x != cp1, d0 = fD[0].x != cp0, d1 = fD[1].x != cp0;
+    const uint2 addA = a0 ? fA[0] : fA[1], addD = d0 ? fD[0] : fD[1];
+    const uint32_t kA = nA > 2 ? 2u : (a0 ? 1u : 0u) + (a1 ? 1u : 0u), kD = nD > 2 ? 2u : (d0 ? 1u : 0u) + (d1 ? 1u : 0u);
     for (uint32_t t0 = 0; t0 < nt && !G.fail; t0 += 32) {
       const uint32_t t = t0 + lane;
       // side 0: a neighbour a of cp0 (its des list), 1: a neighbour d of cp1
@@ -484,19 +455,17 @@ struct WarpGraph {
       const uint32_t ka = side == 0 ? kD : side == 1 ? kA : 0;
       uint32_t n = 0, cap = 0, tot = 0, off = 0;
       if (side >= 0) { n = G.L.nrun[l]; cap = G.L.cap[l]; tot = G.L.total[l]; off = G.L.off[l]; }
-      uint2 ad[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) ad[q] = side == 0 ? addD[q] : addA[q];
-      const bool tiny = side >= 0 && n <= 4 && ka <= 1, small = side >= 0 && n <= 8 && ka <= 2;
+      const uint2 ad = side == 0 ? addD : addA;
+      const bool small = side >= 0 && n <= 8 && ka <= 1;
       // the longer lists' lines on their way into L1
       if (side >= 0 && !small)
         for (uint32_t q = 0; q < n && q < 256; q += 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(G.L.pool + off + q));
       // (mostly a saddle's neighbours or an extremum's saddles: two runs, one added value)
       if (who == 0) {
-        if (!__any_sync(FULL_WARP, small && !tiny)) {
-          if (!lane_edits<4, 1>(tiny, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
+        if (!__any_sync(FULL_WARP, small && n > 4)) {
+          if (!lane_edits<4>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
         } else {
-          if (!lane_edits<8, 2>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
+          if (!lane_edits<8>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
         }
       }
       // the longer lists, each by all lanes of a warp
@@ -506,10 +475,17 @@ struct WarpGraph {
         const int s = __ffs(big) - 1;
         const int bs = __shfl_sync(FULL_WARP, side, s);
         const uint32_t bl = __shfl_sync(FULL_WARP, l, s), bm = __shfl_sync(FULL_WARP, mult, s);
-        const uint32_t bn = __shfl_sync(FULL_WARP, n, s), bc = __shfl_sync(FULL_WARP, cap, s);
-        const uint32_t bt = __shfl_sync(FULL_WARP, tot, s), bo = __shfl_sync(FULL_WARP, off, s);
-        edit_list(bl, bn, bc, bt, bo, bs == 0 ? pD : pA, bs == 0 ? nD : bs == 1 ? nA : 0u, bs == 0 ? cp0 : cp1, bm, true,
-                  bs == 0 || bs == 2 ? cp0 : cp1, bs == 0);
+        uint32_t bn = __shfl_sync(FULL_WARP, n, s), bc = __shfl_sync(FULL_WARP, cap, s);
+        uint32_t bt = __shfl_sync(FULL_WARP, tot, s), bo = __shfl_sync(FULL_WARP, off, s);
+        const uint2 *S = bs == 0 ? pD : pA;
+        uint32_t sn = bs == 0 ? nD : bs == 1 ? nA : 0u;
+        // more added values than the scratch holds: ascending parts, one merge each
+        for (const uint32_t part = (uint32_t)min(G.tmp_cap / 2, 1ull << 30); sn > part && sn > 32 && !G.fail; sn -= part, S += part) {
+          edit_list(bl, bn, bc, bt, bo, S, part, bs == 0 ? cp0 : cp1, bm, false, 0u, bs == 0);
+          bn = G.L.nrun[bl]; bc = G.L.cap[bl]; bt = G.L.total[bl]; bo = G.L.off[bl];
+        }
+        if (!G.fail)
+          edit_list(bl, bn, bc, bt, bo, S, sn, bs == 0 ? cp0 : cp1, bm, true, bs == 0 || bs == 2 ? cp0 : cp1, bs == 0);
       }
     }
   }
@@ -789,6 +765,30 @@ struct WarpGraph {
     if (!off && !G.fail && G.tick(ticks)) set_list(l, b, n);
     drop_scratch(n);
     return !off;
+  }
+
+  // A warp's share of uncancelling the pairs canc[0..npairs) (first the point
+  // whose asc list holds the other), the last one first, asc and des list as
+  // tasks of their own, taken in order from team->ticket (2 * npairs at the
+  // start).  `ord` and `done` are set up for them; the CANCELLED flags stay.
+  __device__ __forceinline__ void uncancel_shared(const uint2 *canc, uint32_t npairs) {
+    for (;;) {
+      unsigned long long t = 0;
+      if (lane == 0) t = atomicAdd(&team->ticket, ~0ull);  // takes one
+      t = __shfl_sync(FULL_WARP, t, 0);
+      if (t == 0 || t > 2ull * npairs) break;  // none left
+      if (__any_sync(FULL_WARP, *(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong)) break;
+      const uint32_t k = (uint32_t)((t - 1) / 2), i = (uint32_t)(t & 1);
+      const uint2 c = canc[k];
+      if (!uncancel_list(c.x, c.y, (int)i, k + 1)) team->wrong = 1;
+      if (G.fail) {
+        team->fail = 1;
+        break;
+      }
+      __threadfence_block();
+      __syncwarp();
+      if (lane == 0) atomicOr(&done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
+    }
   }
 };
 
