@@ -46,6 +46,7 @@ static cudaStream_t pick(dmsc_ctx *c, void *s) { return s ? (cudaStream_t)s : c-
 static int status_to_error(uint32_t st) {
   if (!st) return DMSC_OK;
   if (st & ST_NAN_INPUT) return fail(DMSC_ERR_INPUT, "NaN height in input (outside the supported domain)");
+  if (st & ST_TOO_LONG) return fail(DMSC_ERR_OOM, "lists or discs of more than 2^32 - 1 entries");
   if (st & (ST_RESOLVE_LIMIT | ST_SIMPLIFY_LIMIT))
     return fail(DMSC_ERR_DEVICE_TIMEOUT, "a bounded device loop ran out of iterations (status " + std::to_string(st) + ")");
   return fail(DMSC_ERR_INVARIANT, "device invariant violated (status " + std::to_string(st) + ")");
@@ -421,7 +422,7 @@ int dmsc_msc_simplify_un_simplify(dmsc_msc *m, double tresh, int64_t max_ops, vo
   CK(cudaSetDevice(m->ctx->device));
   cudaStream_t st = pick(m->ctx, stream);
   unsigned long long *hs = nullptr;
-  CK(cudaMallocHost((void **)&hs, sizeof(unsigned long long) * 5));
+  CK(cudaMallocHost((void **)&hs, sizeof(unsigned long long) * 8));
   SimplifyIO io;
   io.ncp = m->ncp; io.nasc = m->nasc; io.ndes = m->ndes;
   io.cellid = m->cellid.p; io.fn = m->fn.p; io.flags = m->flags.p; io.pair_idx = m->pair_idx.p;
@@ -504,7 +505,13 @@ int dmsc_dataset_fill_discs(dmsc_dataset *d, dmsc_msc *m, void *stream) {
   const uint32_t *w[1] = {d->scal.p};
   CK(read_words(d->host_scal, w, 1, st));
   CK(cudaStreamSynchronize(st));
-  if (const uint32_t stw = d->host_scal[0]) return status_to_error(stw);
+  if (io.too_long) {  // no discs
+    m->nadisc = m->nddisc = 0;
+    CK(cudaMemsetAsync(m->adoff.p, 0, 4 * (n + 1), st));
+    CK(cudaMemsetAsync(m->ddoff.p, 0, 4 * (n + 1), st));
+    CK(cudaStreamSynchronize(st));
+  }
+  if (const uint32_t stw = d->host_scal[0] | (io.too_long ? ST_TOO_LONG : 0u)) return status_to_error(stw);
   m->nadisc = io.nadisc;
   m->nddisc = io.nddisc;
   return DMSC_OK;

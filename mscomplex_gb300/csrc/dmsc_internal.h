@@ -62,6 +62,8 @@ cudaError_t scan_exclusive_u32(const uint32_t *in, long long n, uint32_t *out, u
 // dst[0..n) = src[0..n) on the device with a kernel (no copy engine: see
 // read_words)
 cudaError_t copy_u32(uint32_t *dst, const uint32_t *src, long long n, cudaStream_t st);
+// *sum += the sum of a[0..n) in 64 bits (what a 32-bit scan's total would wrap at)
+cudaError_t sum_u32(const uint32_t *a, long long n, unsigned long long *sum, cudaStream_t st);
 // Reads up to 8 device words src[0..n) into host[0..n) with a one-warp kernel
 // that stores into the pinned host memory directly (memory from
 // cudaMallocHost / cudaHostAlloc, which kernels address by the same pointer).
@@ -103,7 +105,7 @@ struct SimplifyIO {
   double tresh = 0;
   unsigned long long max_ops = 0;
   unsigned long long heap_cap = 0, tmp_cap = 0, pool_extra = 0;  // 0 = defaults
-  unsigned long long *host_stats = nullptr;  // [0] pushes [1] pops [2] cancels [3] ops [4] status
+  unsigned long long *host_stats = nullptr;  // pinned, 8 words: [0] pushes [1] pops [2] cancels [3] ops [4] status [5] asc [6] des entries
   long long nasc_out = 0, ndes_out = 0;
   void *work = nullptr;
 };
@@ -158,6 +160,7 @@ struct DiscIO {
   cudaEvent_t ev_place[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // around the saddle-disc placement, per kind, when set
   bool no_cancel = false;  // the complex has no boundary-cancelable critical point
   long long nadisc = 0, nddisc = 0;
+  bool too_long = false;   // a kind's discs have more cells, pieces or chains than 32-bit offsets reach: no discs were written
   // the des discs run on `aux` beside the asc discs on the caller's stream;
   // ev[0]/ev[1] order the two streams; hcounts: 16 words of pinned host memory
   cudaStream_t aux = nullptr;

@@ -271,18 +271,25 @@ cudaError_t mgraph_to_csr(const MGraphHost &h, dmsc_msc &out, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(out.flags.p, m.G.flags, n, cudaMemcpyDeviceToDevice, st);
   }
   for (int w = 0; w < 2 && e == cudaSuccess; ++w) {
-    uint32_t *tot = nullptr;
-    e = cudaMallocAsync((void **)&tot, 4ull * (n + 1), st);
+    uint32_t *tot = nullptr;  // the lists' lengths; before them their sum in 64 bits
+    e = cudaMallocAsync((void **)&tot, 4ull * (n + 1) + 16, st);
     if (e != cudaSuccess) break;
+    unsigned long long *sum = (unsigned long long *)tot, hsum = 0;
+    uint32_t *const buf = tot;
+    tot += 4;
+    e = cudaMemsetAsync(sum, 0, 8, st);
     uint32_t *off = w ? out.doff.p : out.aoff.p;
     if (n) {
       k_mg_totals<<<nblk(n), 256, 0, st>>>(m, w, tot);
       DMSC_LAUNCHED(1);
     }
-    e = scan_exclusive_u32(tot, n, off, off + n, st);
+    if (e == cudaSuccess) e = sum_u32(tot, n, sum, st);
+    if (e == cudaSuccess) e = scan_exclusive_u32(tot, n, off, off + n, st);
     uint32_t total = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total, off + n, 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hsum, sum, 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && hsum > 0xffffffffull) e = cudaErrorMemoryAllocation;  // 32-bit offsets
     DevBuf<uint32_t> &lb = w ? out.des : out.asc;
     if (e == cudaSuccess) e = lb.ensure((size_t)total + 1, st);
     if (e == cudaSuccess && n) {
@@ -291,7 +298,7 @@ cudaError_t mgraph_to_csr(const MGraphHost &h, dmsc_msc &out, cudaStream_t st) {
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) (w ? out.ndes : out.nasc) = total;
-    cudaFreeAsync(tot, st);
+    cudaFreeAsync(buf, st);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e;

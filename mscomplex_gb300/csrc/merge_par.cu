@@ -1444,9 +1444,14 @@ cudaError_t down_child(MGraphHost &hp, const uint32_t *jb, uint32_t njb, unsigne
   if (e == cudaSuccess) e = scan_exclusive_u32(tot_a, n, out.aoff.p, out.aoff.p + n, st);
   if (e == cudaSuccess) e = scan_exclusive_u32(tot_d, n, out.doff.p, out.doff.p + n, st);
   uint32_t tot[2] = {0, 0};
+  unsigned long long *sum = (unsigned long long *)(ctr + 4), hsum[2] = {0, 0};  // the same totals in 64 bits
+  if (e == cudaSuccess) e = sum_u32(tot_a, n, sum, st);
+  if (e == cudaSuccess) e = sum_u32(tot_d, n, sum + 1, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hsum, sum, 16, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&tot[0], out.aoff.p + n, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&tot[1], out.doff.p + n, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && std::max(hsum[0], hsum[1]) > 0xffffffffull) e = cudaErrorMemoryAllocation;  // 32-bit offsets
   if (e == cudaSuccess) e = out.asc.ensure((size_t)tot[0] + 1, st);
   if (e == cudaSuccess) e = out.des.ensure((size_t)tot[1] + 1, st);
   if (e == cudaSuccess && n) {

@@ -279,6 +279,23 @@ cudaError_t copy_u32(uint32_t *dst, const uint32_t *src, long long n, cudaStream
   return cudaGetLastError();
 }
 
+__global__ void k_sum_u32(long long n, const uint32_t *__restrict__ a, unsigned long long *sum) {
+  unsigned long long s = 0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) s += a[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(sum, s);
+}
+
+cudaError_t sum_u32(const uint32_t *a, long long n, unsigned long long *sum, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  long long b = (n + 255) / 256;
+  if (b > 152 * 8) b = 152 * 8;
+  k_sum_u32<<<(unsigned)b, 256, 0, st>>>(n, a, sum);
+  DMSC_LAUNCHED(1);
+  return cudaGetLastError();
+}
+
 struct Words8 {
   const uint32_t *src[8];
 };

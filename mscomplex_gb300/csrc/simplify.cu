@@ -106,7 +106,7 @@ struct SimpArgs {
   bool loose;
   int rx0, ry0, rx1, ry1;  // m_rect of the complex (cell coordinates)
   double tresh;
-  unsigned long long *stats;  // [0] pushes [1] pops [2] cancels [3] ops [4] status
+  unsigned long long *stats;  // [0] pushes [1] pops [2] cancels [3] ops [4] status [5] asc [6] des entries
   // the complex's CSR lists (offsets may be based anywhere) and the entries of
   // its first pushes, one per des arc in that order (k_simp_prep)
   const uint32_t *aoff, *asc, *doff, *des;
@@ -751,6 +751,25 @@ __global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, ui
   }
 }
 
+// The asc and des entries of args[blockIdx.y]'s lists.  Cancellations multiply
+// counts, so a complex of a few thousand points can come to more entries than
+// 32-bit offsets reach; the host refuses it before anything is sized by them.
+__global__ void k_entry_sums(SimpArgs *args) {
+  const SimpArgs &A = args[blockIdx.y];
+  unsigned long long s[2] = {0, 0};
+  const uint2 *tot = reinterpret_cast<const uint2 *>(A.G.L.total);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A.G.ncp; i += gridDim.x * blockDim.x) {
+    const uint2 t = tot[i];
+    s[0] += t.x;
+    s[1] += t.y;
+  }
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    s[w] = warp_sum64(s[w]);
+    if ((threadIdx.x & 31) == 0 && s[w]) atomicAdd(&A.stats[5 + w], s[w]);
+  }
+}
+
 static cudaError_t launch_simplify(SimpArgs *args, int n, int levels, cudaStream_t st) {
   // warps and runs of scratch per block: one block per SM, or several when a batch has more complexes than SMs
   const int warps = n <= 152 ? 16 : 8;
@@ -764,7 +783,8 @@ static cudaError_t launch_simplify(SimpArgs *args, int n, int levels, cudaStream
   if (attr != cudaSuccess) return attr;
   k_simplify<<<n, 32 * SIMP_WARPS, top_bytes(levels), st>>>(args, n, levels);
   k_unsimplify<<<n, 32 * warps, sizeof(uint2) * (warps * own + shared) + sizeof(uint32_t) * DONE_WORDS, st>>>(args, n, own, shared);
-  DMSC_LAUNCHED(2);
+  k_entry_sums<<<dim3(n == 1 ? 64 : 4, n), 256, 0, st>>>(args);
+  DMSC_LAUNCHED(3);
   return cudaGetLastError();
 }
 
@@ -788,16 +808,69 @@ __global__ void k_lists_from_csr(uint32_t ncp, const uint32_t *aoff, const uint3
   }
 }
 
-// run-length lists -> expanded CSR (offsets from a scan of the totals; a
-// list never writes past the next list's offset)
-__global__ void k_csr_from_lists(uint32_t ncp, const uint32_t *off, const uint32_t *nrun, const uint2 *pool, int which,
-                                 const uint32_t *outoff, uint32_t *out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ncp; i += gridDim.x * blockDim.x) {
-    uint32_t l = 2 * i + which, o = outoff[i];
-    const uint32_t end = outoff[i + 1];
-    const uint2 *p = pool + off[l];
-    for (uint32_t k = 0; k < nrun[l]; ++k)
-      for (uint32_t c = 0; c < p[k].y && o < end; ++c) out[o++] = p[k].x;
+// run-length lists -> expanded CSR (offsets from a scan of the totals; a list
+// never writes past the next list's offset).  Counts multiply over a long
+// simplification (42 million entries in lists of 4,000 points on one 256x256
+// field), so the work goes by the entries: a short list is written by its
+// thread, a longer one by its warp, 32 runs at a time, and of those a run of
+// more than FILL_RUN entries in pieces that k_fill writes, a block each (the
+// 42 million entries: 299 ms with a thread per list, 0.5 ms here).
+constexpr uint32_t FILL_RUN = 1024, FILL_PIECE = 16384;
+struct FillPiece {
+  uint32_t value, at, n;
+};
+static size_t fill_room(unsigned long long entries) { return entries / FILL_RUN + 16; }  // pieces: each, or the run it ends, is longer
+__global__ void __launch_bounds__(256) k_csr_from_lists(uint32_t ncp, const uint32_t *off, const uint32_t *nrun, const uint2 *pool, int which,
+                                                        const uint32_t *outoff, uint32_t *out, FillPiece *pieces, uint32_t *npieces, uint32_t room) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < ncp; i0 += step) {
+    const uint32_t i = i0 + lane;
+    uint32_t o = 0, end = 0, n = 0, src = 0;
+    if (i < ncp) {
+      o = outoff[i];
+      end = outoff[i + 1];
+      n = nrun[2 * i + which];
+      src = off[2 * i + which];
+    }
+    const bool small = end - o <= 16;
+    if (small)
+      for (uint32_t k = 0; k < n; ++k) {
+        const uint2 r = pool[src + k];
+        for (uint32_t c = 0; c < r.y && o < end; ++c) out[o++] = r.x;
+      }
+    for (unsigned big = __ballot_sync(FULL_WARP, !small); big; big &= big - 1) {
+      const int s = __ffs(big) - 1;
+      uint32_t at = __shfl_sync(FULL_WARP, o, s);
+      const uint32_t e = __shfl_sync(FULL_WARP, end, s), m = __shfl_sync(FULL_WARP, n, s), p = __shfl_sync(FULL_WARP, src, s);
+      for (uint32_t k0 = 0; k0 < m && at < e; k0 += 32) {
+        uint2 r = make_uint2(0, 0);
+        if (k0 + lane < m) r = pool[p + k0 + lane];
+        uint32_t all;  // (a list's counts add up to its length)
+        const uint32_t x = at + warp_exscan(r.y, lane, all);
+        const uint32_t cnt = x >= e || x < at ? 0u : min(r.y, e - x);
+        if (cnt > FILL_RUN) {  // whole pieces of the run
+          const uint32_t q = (cnt + FILL_PIECE - 1) / FILL_PIECE, w = atomicAdd(npieces, q);
+          for (uint32_t c = 0; c < q && w + c < room; ++c)
+            pieces[w + c] = FillPiece{r.x, x + c * FILL_PIECE, min(FILL_PIECE, cnt - c * FILL_PIECE)};
+        } else if (cnt <= 4) {
+          for (uint32_t c = 0; c < cnt; ++c) out[x + c] = r.x;
+        }
+        for (unsigned mid = __ballot_sync(FULL_WARP, cnt > 4 && cnt <= FILL_RUN); mid; mid &= mid - 1) {
+          const int u = __ffs(mid) - 1;
+          const uint32_t v = __shfl_sync(FULL_WARP, r.x, u), to = __shfl_sync(FULL_WARP, x, u), c1 = __shfl_sync(FULL_WARP, cnt, u);
+          for (uint32_t c = lane; c < c1; c += 32) out[to + c] = v;
+        }
+        at += all;
+      }
+    }
+  }
+}
+__global__ void __launch_bounds__(256) k_fill(const FillPiece *pieces, const uint32_t *npieces, uint32_t room, uint32_t *out) {
+  const uint32_t n = min(*npieces, room);
+  for (uint32_t b = blockIdx.x; b < n; b += gridDim.x) {
+    const FillPiece p = pieces[b];
+    for (uint32_t c = threadIdx.x; c < p.n; c += blockDim.x) out[p.at + c] = p.value;
   }
 }
 __global__ void k_pick_len(uint32_t ncp, const uint32_t *len, int which, uint32_t *out) {
@@ -894,8 +967,10 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
     DMSC_LAUNCHED(2);
     if ((e = launch_simplify(dargs, 1, TOP_LEVELS, st)) != cudaSuccess) return e;
   }
-  e = cudaMemcpyAsync(io.host_stats, a.stats, sizeof(unsigned long long) * 5, cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(io.host_stats, a.stats, sizeof(unsigned long long) * 7, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && io.host_stats[4] == 0 && std::max(io.host_stats[5], io.host_stats[6]) > 0xffffffffull)
+    io.host_stats[4] = ST_TOO_LONG;
   if (e != cudaSuccess || io.host_stats[4] != 0 || !ncp) return e;
   // new CSR offsets (asc, then des) from the list lengths
   for (int which = 0; which < 2 && e == cudaSuccess; ++which) {
@@ -913,15 +988,38 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
   return e;
 }
 
+// The lists of kind `which` (0 asc, 1 des) into out; entries: at most that many.
+static cudaError_t emit_lists(uint32_t ncp, const uint32_t *off, const uint32_t *nrun, const uint2 *pool, int which,
+                              const uint32_t *outoff, uint32_t *out, unsigned long long entries, cudaStream_t st) {
+  const size_t room = entries > FILL_RUN ? fill_room(entries) : 0;  // (no run can be long enough)
+  char *buf = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (room) {
+    if ((e = cudaMallocAsync((void **)&buf, 16 + sizeof(FillPiece) * room, st)) != cudaSuccess) return e;
+    e = cudaMemsetAsync(buf, 0, 4, st);
+  }
+  uint32_t *n = (uint32_t *)buf;
+  FillPiece *pieces = (FillPiece *)(buf + 16);
+  k_csr_from_lists<<<blocks_for(ncp), 256, 0, st>>>(ncp, off, nrun, pool, which, outoff, out, pieces, n, (uint32_t)room);
+  DMSC_LAUNCHED(1);
+  if (room) {
+    k_fill<<<(unsigned)std::min<size_t>(room, 152 * 8), 256, 0, st>>>(pieces, n, (uint32_t)room, out);
+    DMSC_LAUNCHED(1);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (buf) cudaFreeAsync(buf, st);
+  return e;
+}
+
 cudaError_t simplify_emit(SimplifyIO &io, uint32_t *asc, uint32_t *des, cudaStream_t st) {
   SimplifyWork *w = (SimplifyWork *)io.work;
   const uint32_t ncp = (uint32_t)io.ncp;
   if (!w || !ncp) return cudaSuccess;
-  k_csr_from_lists<<<blocks_for(ncp), 256, 0, st>>>(ncp, w->a.G.L.off, w->a.G.L.nrun, w->a.G.L.pool, 0, io.aoff, asc);
-  DMSC_LAUNCHED(1);
-  k_csr_from_lists<<<blocks_for(ncp), 256, 0, st>>>(ncp, w->a.G.L.off, w->a.G.L.nrun, w->a.G.L.pool, 1, io.doff, des);
-  DMSC_LAUNCHED(1);
-  cudaError_t e = cudaMemcpyAsync(w->flags_in, w->a.G.flags, ncp, cudaMemcpyDeviceToDevice, st);
+  const Lists &L = w->a.G.L;
+  cudaError_t e = emit_lists(ncp, L.off, L.nrun, L.pool, 0, io.aoff, asc, (unsigned long long)io.nasc_out, st);
+  if (e == cudaSuccess) e = emit_lists(ncp, L.off, L.nrun, L.pool, 1, io.doff, des, (unsigned long long)io.ndes_out, st);
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpyAsync(w->flags_in, w->a.G.flags, ncp, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->pair_in, w->a.G.pair_idx, 4ull * ncp, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e;
@@ -1079,6 +1177,21 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
     for (int q = 0; q < 5; ++q) io.host_stats[5 * g + q] = 0;
   for (int k = 0; k < ns; ++k)
     for (int q = 0; q < 5; ++q) io.host_stats[5 * which[k] + q] = hs[8 * k + q];
+  // a grid whose lists outgrow 32-bit offsets fails alone; so does every
+  // further one once the batch's lists together would
+  unsigned long long tot[2] = {(unsigned long long)io.nasc, (unsigned long long)io.ndes};
+  for (int k = 0; k < ns; ++k) {
+    const int g = which[k];
+    const unsigned long long na = hs[8 * k + 5], nd = hs[8 * k + 6];
+    const unsigned long long a0 = io.abase[g + 1] - io.abase[g], d0 = io.dbase[g + 1] - io.dbase[g];
+    if (hs[8 * k + 4] != 0) continue;
+    if (tot[0] - a0 + na > 0xffffffffull || tot[1] - d0 + nd > 0xffffffffull) {
+      io.host_stats[5 * g + 4] = ST_TOO_LONG;
+      continue;
+    }
+    tot[0] += na - a0;
+    tot[1] += nd - d0;
+  }
   return cudaSuccess;  // the caller reads the per-grid status
 }
 
@@ -1114,10 +1227,9 @@ cudaError_t simplify_batch_emit(BatchSimplifyIO &io, uint32_t *asc, uint32_t *de
   BatchSimplifyWork *w = (BatchSimplifyWork *)io.work;
   const uint32_t ncp = (uint32_t)io.ncp;
   if (!w || !ncp) return cudaSuccess;
-  k_csr_from_lists<<<blocks_for(ncp), 256, 0, st>>>(ncp, w->off, w->nrun, w->pool, 0, io.aoff, asc);
-  k_csr_from_lists<<<blocks_for(ncp), 256, 0, st>>>(ncp, w->off, w->nrun, w->pool, 1, io.doff, des);
-  DMSC_LAUNCHED(2);
-  return cudaGetLastError();
+  cudaError_t e = emit_lists(ncp, w->off, w->nrun, w->pool, 0, io.aoff, asc, (unsigned long long)io.nasc_out, st);
+  if (e == cudaSuccess) e = emit_lists(ncp, w->off, w->nrun, w->pool, 1, io.doff, des, (unsigned long long)io.ndes_out, st);
+  return e;
 }
 
 void simplify_batch_release(BatchSimplifyIO &io, cudaStream_t st) {
