@@ -15,9 +15,9 @@
 // the extremum discs from runs of one owner along the rows, stably sorted by
 // owner (row-major order is the append order); a stable sort of the
 // cancelled-extremum seeds by saddle; and the saddle discs as interleaved
-// chains (section 4b below) placed window by window, with one thread per
-// saddle that first counts and then writes its breadth-first discs (the
-// output array as the queue) for the few saddles with more than KMAX chains.
+// chains (section 4b below) placed window by window, with one block per saddle
+// that grows its disc level by level (the output array as the queue) for the
+// few saddles with more than KMAX chains.
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 #include "grid_types.h"
@@ -156,12 +156,17 @@ __global__ void k_seed_count(DiscArgs a, int kind, uint32_t *cnt) {
     cnt[i] = c;
   }
 }
-__global__ void k_seed_write(DiscArgs a, int kind, const uint32_t *off, uint32_t *key, uint32_t *val) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.ncp; i += gridDim.x * blockDim.x) {
-    uint32_t o = off[i], e = off[i + 1];
-    if (o == e) continue;
-    const uint32_t *lst = kind ? a.asc + a.aoff[i] : a.des + a.doff[i];
-    for (uint32_t k = 0; k < e - o; ++k) { key[o + k] = lst[k]; val[o + k] = i; }
+// (one thread per item: a cancelled extremum's list may hold most of them)
+__global__ void k_seed_write(DiscArgs a, int kind, const uint32_t *off, uint32_t n, uint32_t *key, uint32_t *val) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    uint32_t lo = 0, hi = a.ncp;  // the last point whose items start at or before p
+    while (hi - lo > 1) {
+      const uint32_t m = lo + (hi - lo) / 2;
+      if (off[m] <= p) lo = m; else hi = m;
+    }
+    const uint32_t *lst = kind ? a.asc + a.aoff[lo] : a.des + a.doff[lo];
+    key[p] = lst[p - off[lo]];
+    val[p] = lo;
   }
 }
 
@@ -170,6 +175,9 @@ struct SeedRuns {
   const uint32_t *val;     // sorted pushers
   const uint32_t *start;   // first sorted position of each saddle (valid when count > 0)
   const uint32_t *count;   // items per saddle
+  const uint32_t *key;     // their saddles
+  const uint32_t *chains;  // exclusive scan over the items of the chains each starts
+  uint32_t n;              // items
 };
 
 // Successors of one path cell (kind 0: asc, via cofacets; kind 1: des, via
@@ -212,69 +220,20 @@ __device__ __forceinline__ int own_seeds(const DiscArgs &a, int kind, uint32_t s
   return n;
 }
 
-// Initial disc vector of saddle s: pushes from cancelled extrema with index
-// < s, then its own seeds, then pushes with index > s.  Calls f(cell).
-template <class F>
-__device__ __forceinline__ void for_seeds(const DiscArgs &a, int kind, uint32_t s, const SeedRuns &sr, F f) {
-  uint32_t cnt = sr.count[s], st = sr.start[s];
-  uint32_t k = 0;
-  for (; k < cnt && sr.val[st + k] < s; ++k) f(a.cellid[a.pair_idx[sr.val[st + k]]]);
-  uint32_t own[4];
-  int n = own_seeds(a, kind, a.cellid[s], own);
-  for (int q = 0; q < n; ++q) f(own[q]);
-  for (; k < cnt; ++k) f(a.cellid[a.pair_idx[sr.val[st + k]]]);
-}
-
-// Serial pass for saddles with more than KMAX chains.  1: disc lengths (every
-// non-critical path cell has at most one successor, so each seed expands into
-// at most two chains).
-__global__ void k_saddle_disc_count(DiscArgs a, int kind, SeedRuns sr, const uint8_t *big, uint32_t *len,
-                                    unsigned long long limit) {
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < a.ncp; s += gridDim.x * blockDim.x) {
-    if (!big[s]) continue;
-    unsigned long long total = 0;
-    bool bad = false;
-    for_seeds(a, kind, s, sr, [&](uint32_t seed) {
-      ++total;
-      uint32_t nx[2];
-      int n = next_cells(a, kind, seed, nx);
-      for (int b = 0; b < n; ++b) {
-        uint32_t c = nx[b];
-        // a gradient path is acyclic: a chain is never longer than `limit` (the cell count)
-        for (unsigned long long steps = 0;; ++steps) {
-          if (steps >= limit) { bad = true; break; }
-          ++total;
-          uint32_t nn[2];
-          int m = next_cells(a, kind, c, nn);
-          if (m == 0) break;
-          if (m > 1) { atomicOr(a.status, ST_INVARIANT); break; }  // a chain cell never branches
-          c = nn[0];
-        }
-      }
-    });
-    if (bad) { atomicOr(a.status, ST_CYCLE); total = 0; }
-    if (total > 0xffffffffull) { atomicOr(a.status, ST_SIMPLIFY_LIMIT); total = 0; }
-    len[s] = (uint32_t)total;
+// The initial disc vector of saddle s: the pushes from cancelled extrema with
+// index < s, then its own seeds, then the pushes with index > s.  Pushes with
+// index < s:
+__device__ __forceinline__ uint32_t pushes_before(const SeedRuns &sr, uint32_t s) {
+  uint32_t lo = 0, hi = sr.count[s];
+  const uint32_t *v = sr.val + (hi ? sr.start[s] : 0);
+  while (lo < hi) {
+    const uint32_t m = (lo + hi) >> 1;
+    if (v[m] < s) lo = m + 1; else hi = m;
   }
+  return lo;
 }
-
-// 2: the reference's breadth-first growth, the output span is the queue
-__global__ void k_saddle_disc_write(DiscArgs a, int kind, SeedRuns sr, const uint8_t *big, const uint32_t *off,
-                                    uint32_t *out) {
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < a.ncp; s += gridDim.x * blockDim.x) {
-    if (!big[s]) continue;
-    uint32_t o = off[s], cap = off[s + 1] - o, tail = 0;
-    uint32_t *q = out + o;
-    for_seeds(a, kind, s, sr, [&](uint32_t seed) { if (tail < cap) q[tail++] = seed; });
-    for (uint32_t head = 0; head < tail; ++head) {
-      uint32_t nx[2];
-      int n = next_cells(a, kind, q[head], nx);
-      for (int b = 0; b < n; ++b) {
-        if (tail < cap) q[tail++] = nx[b];
-        else atomicOr(a.status, ST_INVARIANT);
-      }
-    }
-  }
+__device__ __forceinline__ uint32_t seed_cell(const DiscArgs &a, const SeedRuns &sr, uint32_t p) {
+  return a.cellid[a.pair_idx[sr.val[p]]];
 }
 
 // ---------------------------------------------------------------------------
@@ -298,7 +257,7 @@ __global__ void k_saddle_disc_write(DiscArgs a, int kind, SeedRuns sr, const uin
 // cells of one window of disc positions in shared memory, walking the pieces
 // that reach it one lane each, and stores the window out (k_win_place).
 // ---------------------------------------------------------------------------
-constexpr int KMAX = 32;                 // saddles with more chains take the serial pass
+constexpr int KMAX = 32;                 // saddles with more chains grow level by level (k_big_discs)
 constexpr uint32_t HOP_END = 0xFFFFFFFFu;
 constexpr int HOP_SLOTS = 2 * TX * TY;   // H and Vt edge of every vertex of a tile
 constexpr uint16_t SLOT_NIL = 0xFFFF;
@@ -582,7 +541,9 @@ struct ChainArgs {
   int kind;               // the chains' kind (0 asc, 1 des)
   uint32_t *kc;         // per cp: chains of a saddle handled here (0 otherwise)
   uint32_t *mc;         // per cp: level-0 items
-  uint8_t *big;         // per cp: surviving saddle with more than KMAX chains
+  uint8_t *big;         // per cp: bit 0 a surviving saddle with more than KMAX chains, bits 1-4 the chains of its own seeds, 5-7 those seeds
+  uint32_t *biglist;    // [0] their number, then the saddles with bit 0
+  unsigned long long *dlen;  // per cp: cells of the saddle's disc
   uint32_t *cbase;      // exclusive scan of kc
   uint32_t *cstart, *csaddle, *clen, *cnseg, *csegoff;  // per chain
   uint4 *segs;          // (first edge, first disc position, cells | alive << 8, chain)
@@ -602,56 +563,95 @@ __device__ __forceinline__ int item_children(const DiscArgs &a, int kind, uint32
   return n;
 }
 
+// Work on the items goes by item, not by saddle: after a long simplification
+// one saddle may have millions of them (on one 256x256 field the passes below
+// took 446 ms with a thread per saddle).
+
+// chains that each item starts
+__global__ void k_seed_chains(DiscArgs a, int kind, SeedRuns sr, uint32_t *cnt) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+    const uint32_t s = sr.key[p];
+    uint32_t ch[2];
+    cnt[p] = s < a.ncp && surviving_saddle(a, s) ? (uint32_t)item_children(a, kind, seed_cell(a, sr, p), ch) : 0u;
+  }
+}
+
 __global__ void k_chain_count(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < a.ncp; s += gridDim.x * blockDim.x) {
-    uint32_t m = 0, K = 0;
+    uint32_t m = 0, K = 0, own = 0, ownch = 0;
     if (surviving_saddle(a, s)) {
-      for_seeds(a, kind, s, sr, [&](uint32_t seed) {
-        uint32_t ch[2];
-        ++m;
-        K += item_children(a, kind, seed, ch);
-      });
+      uint32_t seed[4], ch[2];
+      own = (uint32_t)own_seeds(a, kind, a.cellid[s], seed);
+      for (uint32_t q = 0; q < own; ++q) ownch += item_children(a, kind, seed[q], ch);
+      const uint32_t cnt = sr.count[s];
+      m = own + cnt;
+      K = ownch + (cnt ? sr.chains[sr.start[s] + cnt] - sr.chains[sr.start[s]] : 0u);
     }
     const bool big = K > KMAX;
     c.kc[s] = big ? 0 : K;
     c.mc[s] = m;
-    c.big[s] = big;
+    c.big[s] = (uint8_t)((big ? 1u : 0u) | ownch << 1 | own << 5);
+    c.dlen[s] = m;
+    if (big) c.biglist[1 + atomicAdd(c.biglist, 1u)] = s;
   }
 }
 
-// chain starts, lengths and piece counts; the disc length of every saddle
-// handled here (0 for other critical points, big saddles untouched)
-__global__ void k_chain_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c, uint32_t *slen) {
+// The chain from ext-local edge e: its length, stored with its piece count as
+// chain j of saddle s where that saddle's chains are kept.
+__device__ __forceinline__ unsigned long long chain_walk(const DiscArgs &a, const ChainArgs &c, uint32_t s, uint32_t j, uint32_t e) {
+  unsigned long long L = 0;
+  uint32_t nseg = 0;
+  for (uint32_t x = e; x != HOP_END; x = c.hop_to[x]) {
+    const uint32_t l = c.hop_len[x];
+    if (l == 0) { atomicOr(a.status, ST_INVARIANT); break; }  // a chain cell never branches
+    L += l;
+    nseg += (l + SEG_MAX - 1) / SEG_MAX;
+    if (L > c.limit) { atomicOr(a.status, ST_CYCLE); return 0; }
+  }
+  if (!(c.big[s] & 1u)) {
+    // piece slots: one per SEG_MAX cells of each hop, and one more for each level
+    // where another of the saddle's chains ends inside this one (at most K - 1)
+    if (j < c.cap) { c.cstart[j] = e; c.csaddle[j] = s; c.clen[j] = (uint32_t)L; c.cnseg[j] = nseg + c.kc[s] - 1; }
+    else atomicOr(a.status, ST_CAPACITY);
+  }
+  return L;
+}
+// the chains of every saddle's own seeds
+__global__ void k_chain_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < a.ncp; s += gridDim.x * blockDim.x) {
-    if (c.big[s]) continue;
-    if (!surviving_saddle(a, s)) { slen[s] = 0; continue; }
-    unsigned long long total = c.mc[s];
-    uint32_t j = c.cbase[s];
-    bool bad = false;
-    for_seeds(a, kind, s, sr, [&](uint32_t seed) {
+    if (!surviving_saddle(a, s)) continue;
+    const uint32_t kb = pushes_before(sr, s), p0 = sr.count[s] ? sr.start[s] : 0;
+    uint32_t j = c.cbase[s] + (kb ? sr.chains[p0 + kb] - sr.chains[p0] : 0u);
+    uint32_t seed[4], ch[2];
+    const int own = own_seeds(a, kind, a.cellid[s], seed);
+    unsigned long long total = 0;
+    for (int q = 0; q < own; ++q) {
+      const int n = item_children(a, kind, seed[q], ch);
+      for (int b = 0; b < n; ++b) total += chain_walk(a, c, s, j++, ch[b]);
+    }
+    c.dlen[s] += total;
+  }
+}
+// the chains of the items from cancelled extrema
+__global__ void k_seed_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+    const uint32_t s = sr.key[p];
+    unsigned long long total = 0;
+    if (s < a.ncp && surviving_saddle(a, s)) {
+      uint32_t j = c.cbase[s] + sr.chains[p] - sr.chains[sr.start[s]] + (sr.val[p] < s ? 0u : (c.big[s] >> 1) & 15u);
       uint32_t ch[2];
-      const int n = item_children(a, kind, seed, ch);
-      for (int b = 0; b < n; ++b) {
-        unsigned long long L = 0;
-        uint32_t nseg = 0;
-        for (uint32_t e = ch[b]; e != HOP_END; e = c.hop_to[e]) {
-          const uint32_t l = c.hop_len[e];
-          if (l == 0) { atomicOr(a.status, ST_INVARIANT); break; }  // a chain cell never branches
-          L += l;
-          nseg += (l + SEG_MAX - 1) / SEG_MAX;
-          if (L > c.limit) { bad = true; break; }
-        }
-        // piece slots: one per SEG_MAX cells of each hop, and one more for each level
-        // where another of the saddle's chains ends inside this one (at most K - 1)
-        if (j < c.cap) { c.cstart[j] = ch[b]; c.csaddle[j] = s; c.clen[j] = (uint32_t)L; c.cnseg[j] = nseg + c.kc[s] - 1; }
-        else atomicOr(a.status, ST_CAPACITY);
-        ++j;
-        total += L;
-      }
-    });
-    if (bad) { atomicOr(a.status, ST_CYCLE); total = 0; }
-    if (total > 0xffffffffull) { atomicOr(a.status, ST_SIMPLIFY_LIMIT); total = 0; }
-    slen[s] = (uint32_t)total;
+      const int n = item_children(a, kind, seed_cell(a, sr, p), ch);
+      for (int b = 0; b < n; ++b) total += chain_walk(a, c, s, j++, ch[b]);
+    }
+    // items are sorted by saddle: one addition for a warp's items of one saddle
+    const unsigned m = __activemask(), same = __match_any_sync(m, s);
+    if (same == 0xffffffffu) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(m, total, o);
+      if ((threadIdx.x & 31) == 0 && total) atomicAdd(&c.dlen[s], total);
+    } else if (total) {
+      atomicAdd(&c.dlen[s], total);
+    }
   }
 }
 
@@ -730,16 +730,76 @@ __global__ void k_chain_segs(long long nchains, DiscArgs a, ChainArgs c) {
   }
 }
 
-// level-0 items of the saddles handled here
-__global__ void k_level0(DiscArgs a, int kind, SeedRuns sr, ChainArgs c, const uint32_t *off, uint32_t *out) {
+// level-0 items: the saddles' own seeds, and the items from cancelled extrema
+__global__ void k_level0(DiscArgs a, int kind, SeedRuns sr, const uint32_t *off, uint32_t *out) {
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < a.ncp; s += gridDim.x * blockDim.x) {
-    if (c.big[s] || !surviving_saddle(a, s)) continue;
-    uint32_t o = off[s], end = off[s + 1];
-    for_seeds(a, kind, s, sr, [&](uint32_t seed) {
-      if (o < end) out[o++] = seed;
+    if (!surviving_saddle(a, s)) continue;
+    uint32_t seed[4];
+    const int own = own_seeds(a, kind, a.cellid[s], seed);
+    const uint32_t o = off[s] + pushes_before(sr, s), end = off[s + 1];
+    for (int q = 0; q < own; ++q) {
+      if (o + q < end) out[o + q] = seed[q];
       else atomicOr(a.status, ST_INVARIANT);
-    });
+    }
   }
+}
+__global__ void k_seed_level0(DiscArgs a, SeedRuns sr, ChainArgs c, const uint32_t *off, uint32_t *out) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+    const uint32_t s = sr.key[p];
+    if (s >= a.ncp || !surviving_saddle(a, s)) continue;
+    const uint32_t o = off[s] + (p - sr.start[s]) + (sr.val[p] < s ? 0u : c.big[s] >> 5);
+    if (o < off[s + 1]) out[o] = seed_cell(a, sr, p);
+    else atomicOr(a.status, ST_INVARIANT);
+  }
+}
+// Saddles with more than KMAX chains, one block each: the reference's
+// breadth-first growth level by level.  A level is a span of the output; its
+// cells' successors, in order, are the next one.
+constexpr int BIG_THREADS = 256;
+__global__ void __launch_bounds__(BIG_THREADS) k_big_discs(DiscArgs a, int kind, ChainArgs c, const uint32_t *off, uint32_t *out) {
+  __shared__ uint32_t wsum[BIG_THREADS / 32];
+  const uint32_t nbig = c.biglist[0];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t bad = 0;
+  for (uint32_t b = blockIdx.x; b < nbig; b += gridDim.x) {
+    const uint32_t s = c.biglist[1 + b], o = off[s], cap = off[s + 1] - o;
+    uint32_t *q = out + o;
+    unsigned long long lo = 0, hi = c.mc[s];
+    if (hi > cap) { bad = 1; continue; }
+    while (lo < hi) {  // (block-uniform; every level but the last adds cells, at most cap)
+      unsigned long long next = hi;
+      for (unsigned long long base = lo; base < hi; base += BIG_THREADS) {
+        uint32_t nx[2];
+        int n = 0;
+        if (base + threadIdx.x < hi) n = next_cells(a, kind, q[base + threadIdx.x], nx);
+        uint32_t x = (uint32_t)n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+          if (lane >= d) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < BIG_THREADS / 32; ++k) {
+          const uint32_t v = wsum[k];
+          before += k < warp ? v : 0u;
+          all += v;
+        }
+        const unsigned long long at = next + before + x - n;
+        for (int k = 0; k < n; ++k) {
+          if (at + k < cap) q[at + k] = nx[k];
+          else bad = 1;
+        }
+        next += all;
+        __syncthreads();  // wsum is reused; the next level's cells are in place
+      }
+      lo = hi;
+      hi = next < cap ? next : cap;
+    }
+  }
+  if (bad) atomicOr(a.status, ST_INVARIANT);
 }
 
 // Per saddle: the level ranges over which the set of alive chains is
@@ -911,8 +971,21 @@ __global__ void k_run_len(long long n, uint32_t ncp, const uint32_t *key, const 
     }
   }
 }
-__global__ void k_add_counts(uint32_t n, const uint32_t *a, uint32_t *b) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] += a[i];
+// 64-bit sum of every thread's s into *out
+__device__ __forceinline__ void add_sum(unsigned long long s, unsigned long long *out) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
+}
+// b += a, and the sum of the results in 64 bits: the scan of b is 32 bits wide
+__global__ void k_add_counts(uint32_t n, const unsigned long long *a, uint32_t *b, unsigned long long *sum) {
+  unsigned long long s = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned long long v = b[i] + a[i];
+    s += v;
+    b[i] = (uint32_t)v;
+  }
+  add_sum(s, sum);
 }
 // first position of each run of equal sorted keys
 __global__ void k_seed_runs(long long n, uint32_t ncp, const uint32_t *key, uint32_t *start) {
@@ -1074,12 +1147,17 @@ struct DiscKind {
   uint32_t *cnt = nullptr, *slen = nullptr, *sstart = nullptr, *scount = nullptr, *soff = nullptr;
   uint32_t *key = nullptr, *val = nullptr, *kt = nullptr, *vt = nullptr, *kc = nullptr, *mc = nullptr, *cbase = nullptr;
   uint8_t *big = nullptr;
-  uint32_t *hbuf = nullptr;  // pinned host counts: [0] runs, [1] seeds, [2] chains, [3..5] totals
+  uint32_t *hbuf = nullptr;  // pinned host counts: [0] runs, [1] seeds, [2] chains, [3..7] totals
   uint32_t *runbuf = nullptr, *chain_buf = nullptr, *wfirst_buf = nullptr;
   uint4 *segs = nullptr, *blocks = nullptr;
   uint32_t *rp = nullptr, *rstart = nullptr;
   uint32_t nrun = 0, ns = 0, nch = 0, tot[2] = {0, 0};
+  unsigned long long *sums = nullptr;  // disc cells, pieces, chains
+  bool too_long = false;
+  uint32_t *biglist = nullptr;
+  unsigned long long *dlen = nullptr;
   ChainArgs c{};
+  SeedRuns sr{};
   int stage = 0;
   cudaError_t e = cudaSuccess;
 
@@ -1152,7 +1230,7 @@ struct DiscKind {
         ns = hbuf[1];
         if ((long long)ns > S.nmax) { e = cudaErrorInvalidValue; return false; }
         if (ns) {
-          k_seed_write<<<nb(ncp), 256, 0, st>>>(a, kind, soff, key, val);
+          k_seed_write<<<nb(ns), 256, 0, st>>>(a, kind, soff, ns, key, val);
           DMSC_LAUNCHED(1);
           L(radix_sort_pairs(key, val, kt, vt, ns, nbits_for(ncp), st));  // stable: pushers stay in index order
         }
@@ -1164,7 +1242,15 @@ struct DiscKind {
         }
         c.hop_to = S.hop_to; c.hop_len = S.hop_len; c.jseg = S.jseg; c.wcode = S.wcode; c.kind = kind;
         c.kc = kc; c.mc = mc; c.big = big; c.cbase = cbase; c.limit = io.limit;
-        k_chain_count<<<nb(ncp), 128, 0, st>>>(a, kind, SeedRuns{val, sstart, scount}, c);
+        c.biglist = biglist; c.dlen = dlen;
+        L(cudaMemsetAsync(biglist, 0, sizeof(uint32_t), st));
+        sr = SeedRuns{val, sstart, scount, key, vt, ns};
+        if (ns) {  // (the sort's scratch is free again)
+          k_seed_chains<<<nb(ns), 256, 0, st>>>(a, kind, sr, kt);
+          DMSC_LAUNCHED(1);
+          L(scan_exclusive_u32(kt, ns, vt, vt + ns, st));
+        }
+        k_chain_count<<<nb(ncp), 128, 0, st>>>(a, kind, sr, c);
         DMSC_LAUNCHED(1);
         L(scan_exclusive_u32(kc, ncp, cbase, cbase + ncp, st));
         // chain slots: the exact count, or without seeds from cancelled extrema the
@@ -1192,27 +1278,40 @@ struct DiscKind {
         c.cstart = chain_buf; c.csaddle = chain_buf + nch; c.clen = chain_buf + 2 * nch; c.cnseg = chain_buf + 3 * nch;
         c.csegoff = chain_buf + 4 * nch;      // nch + 1
         c.blocks = blocks;
-        const SeedRuns sr{val, sstart, scount};
-        k_chain_len<<<nb(ncp), 128, 0, st>>>(a, kind, sr, c, slen);
-        k_saddle_disc_count<<<nb(ncp), 128, 0, st>>>(a, kind, sr, big, slen, io.limit);
-        k_add_counts<<<nb(ncp), 256, 0, st>>>((uint32_t)ncp, slen, cnt);
-        DMSC_LAUNCHED(3);
+        k_chain_len<<<nb(ncp), 128, 0, st>>>(a, kind, sr, c);
+        DMSC_LAUNCHED(1);
+        if (ns) {
+          k_seed_len<<<nb(ns), 256, 0, st>>>(a, kind, sr, c);
+          DMSC_LAUNCHED(1);
+        }
+        // the disc cells, pieces and chains in 64 bits: more than the offsets reach are refused
+        L(cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * 3, st));
+        k_add_counts<<<nb(ncp), 256, 0, st>>>((uint32_t)ncp, dlen, cnt, sums);
+        DMSC_LAUNCHED(1);
+        L(sum_u32(c.cnseg, nch, sums + 1, st));
+        L(sum_u32(kc, ncp, sums + 2, st));
         uint32_t *offs = kind ? io.ddoff : io.adoff;
         L(scan_exclusive_u32(cnt, ncp, offs, offs + ncp, st));
         L(scan_exclusive_u32(c.cnseg, nch, c.csegoff, c.csegoff + nch, st));
-        const uint32_t *w[2] = {offs + ncp, c.csegoff + nch};
-        L(read_words(&hbuf[3], w, 2, st));
+        const uint32_t *s32 = reinterpret_cast<const uint32_t *>(sums);
+        const uint32_t *w[5] = {offs + ncp, c.csegoff + nch, s32 + 1, s32 + 3, s32 + 5};
+        L(read_words(&hbuf[3], w, 5, st));
         return true;
       }
       case 4: {  // the cells
         for (int q = 0; q < 2; ++q) tot[q] = hbuf[3 + q];
+        if (hbuf[5] | hbuf[6] | hbuf[7]) {
+          too_long = true;
+          tot[0] = tot[1] = 0;
+          release();
+          return false;
+        }
         uint32_t *offs = kind ? io.ddoff : io.adoff;
         DevBuf<uint32_t> *ob = kind ? io.ddisc : io.adisc;
         L(ob->ensure((size_t)tot[0] + 1, st));
         L(cudaMallocAsync((void **)&segs, sizeof(uint4) * ((size_t)tot[1] + 1), st));
         if (e != cudaSuccess) return false;
         c.segs = segs;
-        const SeedRuns sr{val, sstart, scount};
         k_zip_blocks<<<nb(ncp), 128, 0, st>>>(a, c, offs);  // the records the pieces are placed by
         DMSC_LAUNCHED(1);
         if (nch) {
@@ -1222,8 +1321,8 @@ struct DiscKind {
         if (S.io->ev_place[kind][0]) L(cudaEventRecord(S.io->ev_place[kind][0], st));
         if (tot[1] && tot[0]) {
           const uint32_t nwin = (uint32_t)(((unsigned long long)tot[0] + WIN - 1) / WIN);
-          // the window starts reuse the per-saddle disc lengths (slen, ncp words, read
-          // by no later kernel); a complex with fewer critical points than windows allocates
+          // the window starts reuse the seed counts (slen, ncp words, read by no
+          // later kernel); a complex with fewer critical points than windows allocates
           uint32_t *wfirst = nwin <= (uint32_t)ncp ? slen : nullptr;
           if (!wfirst) L(cudaMallocAsync((void **)&wfirst_buf, sizeof(uint32_t) * nwin, st));
           if (e != cudaSuccess) return false;
@@ -1233,9 +1332,13 @@ struct DiscKind {
                                                                                   (unsigned long long)tot[0]);
           DMSC_LAUNCHED(2);
         }
-        k_level0<<<nb(ncp), 128, 0, st>>>(a, kind, sr, c, offs, ob->p);
-        k_saddle_disc_write<<<nb(ncp), 128, 0, st>>>(a, kind, sr, big, offs, ob->p);
-        DMSC_LAUNCHED(2);
+        k_level0<<<nb(ncp), 128, 0, st>>>(a, kind, sr, offs, ob->p);
+        DMSC_LAUNCHED(1);
+        if (ns) {  // (own seeds start at most 8 chains: only with more items are there big saddles)
+          k_seed_level0<<<nb(ns), 256, 0, st>>>(a, sr, c, offs, ob->p);
+          k_big_discs<<<152 * 4, BIG_THREADS, 0, st>>>(a, kind, c, offs, ob->p);
+          DMSC_LAUNCHED(2);
+        }
         // between the two events: every saddle disc cell of this kind is written once
         if (S.io->ev_place[kind][1]) L(cudaEventRecord(S.io->ev_place[kind][1], st));
         if (n > 0 && nrun) {  // extremum discs of this kind
@@ -1271,9 +1374,9 @@ cudaError_t fill_discs(DiscIO &io, cudaStream_t st) {
   const bool seeds = !io.no_cancel;
   // shared words: redir (ncp) | owner keys and run ids 2 (nV + nF) | hops 3 nE
   // per kind: cnt slen sstart scount (4 ncp) soff (ncp + 8) kc mc cbase (3 ncp + 1) big (ncp / 4 + 1)
-  //           seed sort 4 nmax (only with seeds) | pinned counts
-  const size_t kwords = (size_t)ncp * 8 + 16 + (size_t)ncp / 4 + 1 + (seeds ? 4 * (size_t)nmax : 0);
-  size_t words = (size_t)ncp + 8 + (size_t)(nV + nF) * 2 + 2 * (size_t)nE + (size_t)nE / 2 + succ_words(g) / 2 + 64 +
+  //           biglist (ncp + 1) dlen (2 ncp) | seed sort 4 nmax (only with seeds) | pinned counts
+  const size_t kwords = (size_t)ncp * 11 + 32 + (size_t)ncp / 4 + 1 + (seeds ? 4 * (size_t)nmax : 0);
+  size_t words = 16 + (size_t)ncp + 8 + (size_t)(nV + nF) * 2 + 2 * (size_t)nE + (size_t)nE / 2 + succ_words(g) / 2 + 64 +
                  2 * kwords;
   uint32_t *buf = nullptr;
   cudaError_t e = hops_attr();
@@ -1282,6 +1385,7 @@ cudaError_t fill_discs(DiscIO &io, cudaStream_t st) {
   e = cudaMallocAsync((void **)&buf, sizeof(uint32_t) * words, st);
   if (e != cudaSuccess) return e;
   uint32_t *p = buf;
+  uint32_t *sums = p; p += 16;  // (8-byte aligned: the buffer's start)
   S.redir = p; p += ncp + 8;
   S.gkey[0] = p; p += nV;
   S.gkey[1] = p; p += nF;
@@ -1298,6 +1402,7 @@ cudaError_t fill_discs(DiscIO &io, cudaStream_t st) {
     D.st = k ? io.aux : st;
     D.sh = &S;
     D.hbuf = io.hcounts + 8 * k;
+    D.sums = reinterpret_cast<unsigned long long *>(sums) + 3 * k;
     D.cnt = p; p += ncp;
     D.slen = p; p += ncp;
     D.sstart = p; p += ncp;
@@ -1307,6 +1412,9 @@ cudaError_t fill_discs(DiscIO &io, cudaStream_t st) {
     D.mc = p; p += ncp;
     D.cbase = p; p += ncp + 1;
     D.big = (uint8_t *)p; p += ncp / 4 + 1;
+    D.biglist = p; p += ncp + 1;
+    p += (p - buf) & 1;  // 8-byte aligned
+    D.dlen = (unsigned long long *)p; p += 2 * ncp;
     if (seeds) {
       D.key = p; p += nmax;
       D.val = p; p += nmax;
@@ -1351,6 +1459,7 @@ cudaError_t fill_discs(DiscIO &io, cudaStream_t st) {
     for (int k = 0; k < 2; ++k) {
       if (K[k].e != cudaSuccess && e == cudaSuccess) e = K[k].e;
       K[k].release();
+      io.too_long |= K[k].too_long;
     }
     io.nadisc = K[0].tot[0];
     io.nddisc = K[1].tot[0];

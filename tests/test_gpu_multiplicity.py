@@ -1,5 +1,6 @@
 """Cancellations multiply the counts of the asc / des multisets: lists of
-thousands of equal entries, and fields whose lists outgrow 32-bit offsets.  Noisy bumps at 5% of their range."""
+thousands of equal entries, saddles with thousands of disc items, and fields
+whose lists outgrow 32-bit offsets.  Noisy bumps at 5% of their range."""
 import numpy as np
 import pytest
 
@@ -21,6 +22,19 @@ def simplified(M, f, tresh=0.05):
     m = ds.writeout_connectivity()
     m.simplify_un_simplify(tresh)
     return ds, m
+
+
+@pytest.mark.parametrize("n,seed", [(96, 12), (96, 20), (96, 4), (96, 10), (128, 19)])
+def test_saddles_with_many_disc_items(gpu_lib, oracle, n, seed):
+    """Up to 57, 132, 937, 4019 and 1180 items from cancelled extrema at one
+    saddle: its chains around and past the 32 that are interleaved, and levels
+    around and past a block's threads."""
+    f = noisy_bumps(n, seed)
+    r = full_rect(f)
+    want = oracle.Dataset(f, r, r, tresh=0.05, fill_discs=True).msc()
+    ds, m = simplified(gpu_lib, f)
+    ds.post_merge_fill_discs(m)
+    assert_same_complex(m.export(), want, f"{n} seed {seed}")
 
 
 @pytest.mark.parametrize("seed", [231, 236, 391])
