@@ -48,6 +48,7 @@ struct TeamState {
   int lock;                  // 1: a warp uses the scratch all warps share
 };
 constexpr unsigned long long WAIT_LIMIT = 1ull << 26;  // polls of a wait on another warp
+constexpr int BAR_EDIT = 3;
 
 struct WarpGraph {
   Graph G;        // the same in every lane
@@ -423,7 +424,10 @@ struct WarpGraph {
     }
   }
   // The edits of all neighbours' lists, by warp `who` of `warps`: the short
-  // lists by warp 0, the longer ones in turn.
+  // lists by warp 0, the longer ones in turn.  Every warp sorts the lists into
+  // short and long by their lengths, so none of them is edited before all
+  // warps have read its length (barrier BAR_EDIT of those warps, once per 32
+  // neighbours: no warp leaves early).
   __device__ __forceinline__ void edit_neighbours(const Pair &q, int who, int warps) {
     const uint32_t cp0 = q.cp0, cp1 = q.cp1;
     const uint2 o0 = q.o0, o1 = q.o1;
@@ -442,7 +446,7 @@ struct WarpGraph {
     const bool a0 = fA[0].x != cp1, a1 = fA[1].x != cp1, d0 = fD[0].x != cp0, d1 = fD[1].x != cp0;
     const uint2 addA = a0 ? fA[0] : fA[1], addD = d0 ? fD[0] : fD[1];
     const uint32_t kA = nA > 2 ? 2u : (a0 ? 1u : 0u) + (a1 ? 1u : 0u), kD = nD > 2 ? 2u : (d0 ? 1u : 0u) + (d1 ? 1u : 0u);
-    for (uint32_t t0 = 0; t0 < nt && !G.fail; t0 += 32) {
+    for (uint32_t t0 = 0; t0 < nt; t0 += 32) {
       const uint32_t t = t0 + lane;
       // side 0: a neighbour a of cp0 (its des list), 1: a neighbour d of cp1
       // (its asc list), 2 / 3: an erase from an asc / a des list only
@@ -457,16 +461,18 @@ struct WarpGraph {
       if (side >= 0) { n = G.L.nrun[l]; cap = G.L.cap[l]; tot = G.L.total[l]; off = G.L.off[l]; }
       const uint2 ad = side == 0 ? addD : addA;
       const bool small = side >= 0 && n <= 8 && ka <= 1;
+      if (warps > 1) {
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;" ::"r"(BAR_EDIT), "r"(32 * warps) : "memory");
+      }
+      if (G.fail) continue;
       // the longer lists' lines on their way into L1
       if (side >= 0 && !small)
         for (uint32_t q = 0; q < n && q < 256; q += 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(G.L.pool + off + q));
       // (mostly a saddle's neighbours or an extremum's saddles: two runs, one added value)
       if (who == 0) {
-        if (!__any_sync(FULL_WARP, small && n > 4)) {
-          if (!lane_edits<4>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
-        } else {
-          if (!lane_edits<8>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0)) return;
-        }
+        if (!__any_sync(FULL_WARP, small && n > 4)) lane_edits<4>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0);
+        else lane_edits<8>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0);
       }
       // the longer lists, each by all lanes of a warp
       for (unsigned big = __ballot_sync(FULL_WARP, side >= 0 && !small); big && !G.fail; big &= big - 1) {

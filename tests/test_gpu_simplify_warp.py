@@ -50,6 +50,17 @@ def test_long_neighbour_lists(gpu_lib, oracle, hubs):
     simplified(gpu_lib, oracle, f.astype(np.float32), 0.02, f"{hubs} hubs")
 
 
+@pytest.mark.parametrize("y,x,n", [(0, 0, 512), (512, 512, 512), (1024, 0, 400), (0, 2048, 400)])
+def test_quantised_windows(gpu_lib, oracle, y, x, n):
+    """Windows of the 4096x4096 quantised field: thousands of cancellations
+    among lists whose lengths cross the line between short and long."""
+    from mscomplex_gb300 import synth
+    if not hasattr(test_quantised_windows, "field"):
+        test_quantised_windows.field = synth.bumps4096q()
+    f = np.ascontiguousarray(test_quantised_windows.field[y:y + n, x:x + n])
+    simplified(gpu_lib, oracle, f, 0.01, f"window {y},{x} {n}")
+
+
 @pytest.mark.parametrize("count", [152, 153, 330])
 def test_batches_around_one_complex_per_sm(gpu_lib, oracle, count):
     """Up to 152 complexes take the launch shape of a single one, more take the
