@@ -1,13 +1,10 @@
-// primitives.cu -- device-wide exclusive scan, stable LSD radix sort and the
-// kernels that assemble the Morse-Smale complex in CSR form.
+// primitives.cu -- device-wide exclusive scan and the kernels that assemble the
+// Morse-Smale complex in CSR form.
 //
 // The reference's scan is the OpenCL PrefixScan (dmsc/src/prefix_scan.cpp:
-// 340-465, kernels absent: dmsc/resources/scan_kernel.cl is empty) and its
-// sort slot is an unused bitonic sort (dmsc/src/bitonic_sort.cpp).  Both are
-// written here from scratch: the scan is a single pass with decoupled
-// look-back out of place (bounded waits on earlier tiles) and reduce-then-scan
-// in place, the radix sort is a stable 8-bit LSD sort (histogram, scan,
-// match_any-ranked scatter).
+// 340-465, kernels absent: dmsc/resources/scan_kernel.cl is empty).  It is
+// written here from scratch: the sums of equal chunks, one chunk per block,
+// then every block's scan of its chunk.
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 
@@ -117,107 +114,136 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const T *in, long lo
   if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = (block_off ? block_off[blockIdx.x] : 0u) + tot;
 }
 
-// Single-pass scan (decoupled look-back): a block takes the next tile from
-// an atomic counter, publishes its tile's sum, then warp 0 walks back over
-// the earlier tiles' published words -- adding sums until it meets a tile
-// that has published its inclusive prefix -- and publishes its own.  Tiles
-// are taken in counter order, so a block only waits for blocks that already
-// run.  A word is (flag << 32 | value) in one 64-bit store: 0 not yet, 1 the
-// tile's sum, 2 its inclusive prefix.  The wait is bounded: past
-// LOOKBACK_LIMIT polls the block sums the earlier tiles' inputs itself (the
-// same prefix, slower), which is why the input must not be the output.
-constexpr unsigned long long LOOKBACK_LIMIT = 1ull << 22;
-__device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p) {
-  return *reinterpret_cast<const volatile unsigned long long *>(p);
+// Four items at p + 4 * lane of a warp's 128: one vector load per lane, the
+// warp's lanes side by side.
+template <typename T>
+__device__ __forceinline__ void load4(const T *in, long long at, long long n, bool vec, uint32_t v[4]) {
+  if (vec && at + 4 <= n) {
+    if constexpr (sizeof(T) == 4) {
+      const uint4 a = *reinterpret_cast<const uint4 *>(in + at);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+      const uint32_t a = *reinterpret_cast<const uint32_t *>(in + at);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = (a >> (8 * k)) & 0xffu;
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = at + k < n ? (uint32_t)in[at + k] : 0u;
 }
-__device__ __forceinline__ void st_word(unsigned long long *p, unsigned long long v) {
-  *reinterpret_cast<volatile unsigned long long *>(p) = v;
+// The scan of more than one tile: the array is split into one chunk of whole
+// tiles per block, a first launch sums the chunks, and in a second one every
+// block adds up the sums before its own and scans its chunk tile by tile (the
+// second read comes from L2 up to some 25 million items).  No block waits for
+// another: a single pass with decoupled look-back read the items once but
+// spent its time walking back over the tiles in flight (2^24 items: 57 us,
+// here 31; 8 bytes an item are 20 us).  A tile is 16 items a thread: each warp
+// owns 512 consecutive items in four rounds of 128, so that every load and
+// store instruction moves 512 consecutive bytes, and the next tile's loads are
+// issued before the current one is scanned.  In and out may be the same array.
+constexpr int ONE_ROUNDS = 4, ONE_CHUNK = SCAN_THREADS * 4 * ONE_ROUNDS, SCAN_BLOCKS = 152 * 2;
+template <typename T>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const T *__restrict__ in, long long n, bool vec, long long chunk,
+                                                            uint32_t *__restrict__ part) {
+  __shared__ uint32_t red[SCAN_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long b0 = blockIdx.x * chunk, b1 = b0 + chunk < n ? b0 + chunk : n;
+  uint32_t acc = 0;
+  for (long long base = b0 + (long long)warp * (128 * ONE_ROUNDS) + 4 * lane; base < b1; base += ONE_CHUNK) {
+    uint32_t v[ONE_ROUNDS][4];
+#pragma unroll
+    for (int r = 0; r < ONE_ROUNDS; ++r) load4(in, base + 128 * r, b1, vec, v[r]);
+#pragma unroll
+    for (int r = 0; r < ONE_ROUNDS; ++r) acc += v[r][0] + v[r][1] + v[r][2] + v[r][3];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) red[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t s = 0;
+#pragma unroll
+    for (int w = 0; w < SCAN_THREADS / 32; ++w) s += red[w];
+    part[blockIdx.x] = s;
+  }
 }
 template <typename T>
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_onepass(const T *__restrict__ in, long long n, bool vec_in,
-                                                               uint32_t *__restrict__ out, bool vec_out,
-                                                               unsigned long long *__restrict__ word,
-                                                               uint32_t *__restrict__ counter, long long nb,
-                                                               uint32_t *__restrict__ total) {
-  __shared__ uint32_t tile_s, excl_s;
-  if (threadIdx.x == 0) tile_s = atomicAdd(counter, 1u);
-  __syncthreads();
-  const long long tile = tile_s;
-  if (tile >= nb) return;  // (block-uniform)
-  const long long base = tile * SCAN_CHUNK + (long long)threadIdx.x * SCAN_ITEMS;
-  uint32_t v[SCAN_ITEMS];
-  load_items(in, base, n, vec_in, v);
-  uint32_t s = 0;
+__global__ void __launch_bounds__(SCAN_THREADS, 2) k_scan_chunks(const T *in, long long n, bool vec_in, uint32_t *out, bool vec_out,
+                                                                 long long chunk, const uint32_t *__restrict__ part, uint32_t *total) {
+  __shared__ uint32_t wtot[2][SCAN_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long b0 = blockIdx.x * chunk, b1 = b0 + chunk < n ? b0 + chunk : n;
+  const long long at0 = b0 + (long long)warp * (128 * ONE_ROUNDS) + 4 * lane;
+  uint32_t v[ONE_ROUNDS][4], nx[ONE_ROUNDS][4];
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
-  uint32_t ex;
-  const uint32_t tot = block_exscan(s, ex);
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    uint32_t excl = 0;
-    bool fallback = false;
-    if (tile == 0) {
-      if (lane == 0) st_word(word, (2ull << 32) | tot);
-    } else {
-      if (lane == 0) st_word(word + tile, (1ull << 32) | tot);
-      long long j = tile - 1;
-      unsigned long long polls = 0;
-      for (;;) {
-        const long long idx = j - lane;  // lane 0: the nearest earlier tile
-        const unsigned long long w = idx >= 0 ? ld_word(word + idx) : (2ull << 32);
-        const uint32_t flag = (uint32_t)(w >> 32);
-        const unsigned pm = __ballot_sync(0xffffffffu, flag == 2u), zm = __ballot_sync(0xffffffffu, flag == 0u);
-        const int fp = pm ? __ffs(pm) - 1 : 32;  // the nearest tile with its prefix
-        const unsigned need = fp >= 31 ? 0xffffffffu : ((2u << fp) - 1u);
-        if (zm & need) {  // a tile before it has published nothing yet
-          if (++polls > LOOKBACK_LIMIT) { fallback = true; break; }
-          continue;
-        }
-        uint32_t c = lane <= fp ? (uint32_t)w : 0u;
+  for (int r = 0; r < ONE_ROUNDS; ++r) load4(in, at0 + 128 * r, b1, vec_in, nx[r]);
+  uint32_t prefix = 0;  // the items before the tile
+  if (part) {
+    uint32_t s = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) s += part[i];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        excl += c;
-        if (fp < 32) break;
-        j -= 32;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) wtot[1][warp] = s;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < SCAN_THREADS / 32; ++w) prefix += wtot[1][w];
+  }
+  int slot = 0;
+  for (long long tile = b0; tile < b1; tile += ONE_CHUNK, slot ^= 1) {
+    const long long base = at0 + (tile - b0);
+    uint32_t x[ONE_ROUNDS], s[ONE_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < ONE_ROUNDS; ++r) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[r][k] = nx[r][k];
+      x[r] = s[r] = v[r][0] + v[r][1] + v[r][2] + v[r][3];
+    }
+    if (tile + ONE_CHUNK < b1) {
+#pragma unroll
+      for (int r = 0; r < ONE_ROUNDS; ++r) load4(in, base + ONE_CHUNK + 128 * r, b1, vec_in, nx[r]);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int r = 0; r < ONE_ROUNDS; ++r) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x[r], o);
+        if (lane >= o) x[r] += y;
       }
-      fallback = __any_sync(0xffffffffu, fallback);
-      if (!fallback && lane == 0) st_word(word + tile, (2ull << 32) | (excl + tot));
+    uint32_t run = 0;  // x becomes the warp's items before the lane's of the round
+#pragma unroll
+    for (int r = 0; r < ONE_ROUNDS; ++r) {
+      const uint32_t all = __shfl_sync(0xffffffffu, x[r], 31);
+      x[r] += run - s[r];
+      run += all;
     }
-    if (lane == 0) excl_s = fallback ? 0xFFFFFFFFu : excl;
-  }
-  __syncthreads();
-  uint32_t prefix = excl_s;
-  if (prefix == 0xFFFFFFFFu && tile > 0) {  // bounded wait ran out: the earlier tiles' sum from their inputs
-    __shared__ uint32_t red[32];
-    const long long upto = tile * SCAN_CHUNK;
-    uint32_t acc = 0;
-    for (long long i = threadIdx.x; i < upto; i += blockDim.x) acc += (uint32_t)in[i];
+    if (lane == 0) wtot[slot][warp] = run;
+    __syncthreads();  // (one barrier a tile: the slots alternate)
+    uint32_t tot = 0, before = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      uint32_t r = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0u;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-      if (threadIdx.x == 0) { excl_s = r; st_word(word + tile, (2ull << 32) | (r + tot)); }
+    for (int w = 0; w < SCAN_THREADS / 32; ++w) {
+      const uint32_t t = wtot[slot][w];
+      before += w < warp ? t : 0u;
+      tot += t;
     }
-    __syncthreads();
-    prefix = excl_s;
-  }
-  uint32_t run = prefix + ex;
-  uint32_t o[SCAN_ITEMS];
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) { o[k] = run; run += v[k]; }
-  if (vec_out && base + SCAN_ITEMS <= n) {
-    reinterpret_cast<uint4 *>(out + base)[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    reinterpret_cast<uint4 *>(out + base)[1] = make_uint4(o[4], o[5], o[6], o[7]);
-  } else {
+    for (int r = 0; r < ONE_ROUNDS; ++r) {
+      const long long at = base + 128 * r;
+      uint32_t o[4];
+      o[0] = prefix + before + x[r];
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-      if (base + k < n) out[base + k] = o[k];
+      for (int k = 1; k < 4; ++k) o[k] = o[k - 1] + v[r][k - 1];
+      if (vec_out && at + 4 <= b1) {
+        *reinterpret_cast<uint4 *>(out + at) = make_uint4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (at + k < b1) out[at + k] = o[k];
+      }
+    }
+    prefix += tot;
   }
-  if (total && tile == nb - 1 && threadIdx.x == 0) *total = prefix + tot;
+  if (total && b1 == n && threadIdx.x == 0) *total = prefix;
 }
 
 template <typename T>
@@ -226,39 +252,20 @@ cudaError_t scan_exclusive_t(const T *in, long long n, uint32_t *out, uint32_t *
     if (total) return cudaMemsetAsync(total, 0, sizeof(uint32_t), st);
     return cudaSuccess;
   }
-  long long nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  if (nb == 1) {
-    k_scan_down<T><<<1, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), nullptr, out, items_aligned(out), total);
-    DMSC_LAUNCHED(1);
-    return cudaGetLastError();
-  }
-  if ((const void *)in != (const void *)out) {  // one pass (the look-back's fallback reads the input)
-    unsigned long long *word = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&word, sizeof(unsigned long long) * (nb + 1), st);
+  const bool vi = (uintptr_t)in % (4 * sizeof(T)) == 0, vo = (uintptr_t)out % 16 == 0;
+  const long long nt = (n + ONE_CHUNK - 1) / ONE_CHUNK, per = (nt + SCAN_BLOCKS - 1) / SCAN_BLOCKS;  // tiles, and per block
+  const long long chunk = per * ONE_CHUNK, nb = (nt + per - 1) / per;
+  uint32_t *part = nullptr;
+  if (nb > 1) {
+    const cudaError_t e = cudaMallocAsync((void **)&part, sizeof(uint32_t) * nb, st);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(word, 0, sizeof(unsigned long long) * (nb + 1), st);
-    if (e == cudaSuccess) {
-      k_scan_onepass<T><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), out, items_aligned(out), word,
-                                                                reinterpret_cast<uint32_t *>(word + nb), nb, total);
-      DMSC_LAUNCHED(1);
-      e = cudaGetLastError();
-    }
-    cudaFreeAsync(word, st);
-    return e;
-  }
-  uint32_t *part = nullptr, *poff = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&part, sizeof(uint32_t) * nb * 2, st);
-  if (e != cudaSuccess) return e;
-  poff = part + nb;
-  k_scan_reduce<T><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), part);
-  DMSC_LAUNCHED(1);
-  e = scan_exclusive_t<uint32_t>(part, nb, poff, nullptr, st);
-  if (e == cudaSuccess) {
-    k_scan_down<T><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), poff, out, items_aligned(out), total);
+    k_scan_sums<T><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, vi, chunk, part);
     DMSC_LAUNCHED(1);
-    e = cudaGetLastError();
   }
-  cudaFreeAsync(part, st);
+  k_scan_chunks<T><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, vi, out, vo, chunk, part, total);
+  DMSC_LAUNCHED(1);
+  const cudaError_t e = cudaGetLastError();
+  if (part) cudaFreeAsync(part, st);
   return e;
 }
 
@@ -347,179 +354,6 @@ cudaError_t scan_exclusive_u32_scratch(const uint32_t *in, long long n, uint32_t
                                                                 items_aligned(out), total);
   DMSC_LAUNCHED(1);
   return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// stable LSD radix sort of (key, value) pairs on key bits [0, nbits)
-// ---------------------------------------------------------------------------
-constexpr int RS_THREADS = 256;
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ROUNDS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;  // each warp owns a contiguous run of 256 items
-
-__global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const uint32_t *__restrict__ keys, long long n, int shift,
-                                                           uint32_t *__restrict__ hist, long long nb) {
-  __shared__ uint32_t cnt[256];
-  cnt[threadIdx.x] = 0;
-  __syncthreads();
-  long long base = (long long)blockIdx.x * RS_TILE;
-  for (int k = threadIdx.x; k < RS_TILE; k += RS_THREADS) {
-    long long i = base + k;
-    if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[(long long)threadIdx.x * nb + blockIdx.x] = cnt[threadIdx.x];
-}
-
-__global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
-                                                              long long n, int shift, const uint32_t *__restrict__ hoff,
-                                                              long long nb, uint32_t *__restrict__ kout,
-                                                              uint32_t *__restrict__ vout) {
-  __shared__ uint32_t wcnt[RS_WARPS][256];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = threadIdx.x; k < RS_WARPS * 256; k += RS_THREADS) (&wcnt[0][0])[k] = 0;
-  __syncthreads();
-  long long base = (long long)blockIdx.x * RS_TILE + warp * (32 * RS_ROUNDS);
-  uint32_t key[RS_ROUNDS], val[RS_ROUNDS], rank[RS_ROUNDS];
-  const uint32_t lt_mask = (1u << lane) - 1u;
-#pragma unroll
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-    long long i = base + r * 32 + lane;
-    bool valid = i < n;
-    key[r] = valid ? kin[i] : 0u;
-    val[r] = valid ? vin[i] : 0u;
-    uint32_t d = valid ? ((key[r] >> shift) & 255u) : 256u;
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t before = valid ? wcnt[warp][d] : 0u;
-    rank[r] = before + __popc(peers & lt_mask);
-    __syncwarp();
-    if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
-  }
-  __syncthreads();
-  {
-    uint32_t d = threadIdx.x, run = 0;
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; ++w) { uint32_t t = wcnt[w][d]; wcnt[w][d] = run; run += t; }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-    long long i = base + r * 32 + lane;
-    if (i < n) {
-      uint32_t d = (key[r] >> shift) & 255u;
-      uint32_t pos = hoff[(long long)d * nb + blockIdx.x] + wcnt[warp][d] + rank[r];
-      kout[pos] = key[r];
-      vout[pos] = val[r];
-    }
-  }
-}
-
-// Sorts in place (keys/vals) using caller scratch of the same size.
-cudaError_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *ktmp, uint32_t *vtmp, long long n, int nbits,
-                             cudaStream_t st) {
-  if (n <= 1 || nbits <= 0) return cudaSuccess;
-  long long nb = (n + RS_TILE - 1) / RS_TILE;
-  uint32_t *hist = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&hist, sizeof(uint32_t) * 256 * nb * 2, st);
-  if (e != cudaSuccess) return e;
-  uint32_t *hoff = hist + 256 * nb;
-  uint32_t *ka = keys, *va = vals, *kb = ktmp, *vb = vtmp;
-  for (int shift = 0; shift < nbits; shift += 8) {
-    k_radix_hist<<<(unsigned)nb, RS_THREADS, 0, st>>>(ka, n, shift, hist, nb);
-    DMSC_LAUNCHED(1);
-    e = scan_exclusive_u32(hist, 256 * nb, hoff, nullptr, st);
-    if (e != cudaSuccess) break;
-    k_radix_scatter<<<(unsigned)nb, RS_THREADS, 0, st>>>(ka, va, n, shift, hoff, nb, kb, vb);
-    DMSC_LAUNCHED(1);
-    std::swap(ka, kb);
-    std::swap(va, vb);
-  }
-  if (e == cudaSuccess && ka != keys) {
-    e = copy_u32(keys, ka, n, st);
-    if (e == cudaSuccess) e = copy_u32(vals, va, n, st);
-  }
-  cudaFreeAsync(hist, st);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
-}
-
-// Batched key/value sort (the BitonicSortProgram slot): arrays [b*len, (b+1)*len)
-// sorted independently, ascending or descending, stably.  Implemented as one
-// stable LSD sort on the (possibly inverted) key followed by a stable sort on
-// the array index.
-__global__ void k_sort_prepare(long long n, uint32_t len, uint32_t dir, const uint32_t *__restrict__ ks,
-                               const uint32_t *__restrict__ vs, uint32_t *__restrict__ k, uint32_t *__restrict__ v,
-                               uint32_t *__restrict__ seg) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    uint32_t key = ks[i];
-    k[i] = dir ? key : ~key;
-    v[i] = vs[i];
-    seg[i] = (uint32_t)(i / len);
-  }
-}
-__global__ void k_sort_finish(long long n, uint32_t dir, const uint32_t *__restrict__ k, uint32_t *__restrict__ kout) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    kout[i] = dir ? k[i] : ~k[i];
-}
-// (seg, key) pairs: after sorting by key, a stable sort by segment keeps the
-// key order inside each segment.  Values travel through an index permutation.
-__global__ void k_gather_u32(long long n, const uint32_t *__restrict__ idx, const uint32_t *__restrict__ src,
-                             uint32_t *__restrict__ dst) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = src[idx[i]];
-}
-__global__ void k_iota(long long n, uint32_t *__restrict__ a) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    a[i] = (uint32_t)i;
-}
-
-static unsigned grid_for(long long n, int threads);
-
-cudaError_t sort_pairs_batched(uint32_t *dk, uint32_t *dv, const uint32_t *sk, const uint32_t *sv, uint32_t batch,
-                               uint32_t len, uint32_t dir, cudaStream_t st) {
-  long long n = (long long)batch * len;
-  if (n == 0) return cudaSuccess;
-  uint32_t *buf = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&buf, sizeof(uint32_t) * n * 7, st);
-  if (e != cudaSuccess) return e;
-  uint32_t *k = buf, *v = buf + n, *seg = buf + 2 * n, *perm = buf + 3 * n, *t1 = buf + 4 * n, *t2 = buf + 5 * n,
-           *t3 = buf + 6 * n;
-  unsigned gb = grid_for(n, 256);
-  k_sort_prepare<<<gb, 256, 0, st>>>(n, len, dir, sk, sv, k, v, seg);
-  DMSC_LAUNCHED(1);
-  k_iota<<<gb, 256, 0, st>>>(n, perm);
-  DMSC_LAUNCHED(1);
-  // 1) stable by key, carrying the original index
-  e = radix_sort_pairs(k, perm, t1, t2, n, 32, st);
-  if (e == cudaSuccess && batch > 1) {
-    // 2) stable by segment of the original index: seg of perm[i]
-    k_gather_u32<<<gb, 256, 0, st>>>(n, perm, seg, t3);
-    DMSC_LAUNCHED(1);
-    int sbits = 1;
-    while ((1ll << sbits) < (long long)batch) ++sbits;
-    // sort (segment, position-in-key-order) carrying the key-sorted position
-    k_iota<<<gb, 256, 0, st>>>(n, t1);
-    DMSC_LAUNCHED(1);
-    e = radix_sort_pairs(t3, t1, seg, t2, n, sbits, st);
-    if (e == cudaSuccess) {
-      k_gather_u32<<<gb, 256, 0, st>>>(n, t1, k, t2);  // keys in final order
-      DMSC_LAUNCHED(1);
-      k_gather_u32<<<gb, 256, 0, st>>>(n, t1, perm, t3);  // original indices in final order
-      DMSC_LAUNCHED(1);
-      e = copy_u32(k, t2, n, st);
-      if (e == cudaSuccess) e = copy_u32(perm, t3, n, st);
-    }
-  }
-  if (e == cudaSuccess) {
-    k_gather_u32<<<gb, 256, 0, st>>>(n, perm, v, t2);  // values (v holds the source values)
-    DMSC_LAUNCHED(1);
-    k_sort_finish<<<gb, 256, 0, st>>>(n, dir, k, dk);
-    DMSC_LAUNCHED(1);
-    e = copy_u32(dv, t2, n, st);
-  }
-  cudaFreeAsync(buf, st);
-  return e;
 }
 
 // ---------------------------------------------------------------------------
