@@ -571,7 +571,7 @@ enum SeqKind : int { SEQ_UP_CANCEL = 0, SEQ_DOWN_BOUNDARY = 1 };
 struct SeqJob {
   int kind, g0;
   CRect ixn;
-  int win = 0, min_commits = 0;  // SEQ_UP_CANCEL: rounds window (0: one thread) and hand-off rate
+  int win = 0, min_commits = 0;  // SEQ_UP_CANCEL: rounds window (0: groups of cells) and hand-off rate
 };
 
 // Loads, across the GPU, what the one-thread step of a job will read -- the
@@ -613,8 +613,19 @@ __global__ void k_seq_prefetch(const MGraph *graphs, const SeqJob *jobs, uint32_
   if (acc == 0x9E3779B9u && sink) *sink = acc;
 }
 
-// merge_up's boundary cancellations, one job per block.  The first warp walks
-// the boundary cells in the loop's order, 32 at a time: their lanes look the
+// merge_up's boundary cancellations.  A cancellation reads and writes the lists
+// of its two points and of their neighbours, and adds edges among those alone;
+// so cells whose pairs' points and neighbours are joined, over the whole
+// boundary, by no chain of common points never meet, and each such group can be
+// taken on its own, in the loop's order within it.  On white noise most groups
+// are a few cells long (2048^2 cut in two: 2,400 cancellations, the longest group
+// 220); where one extremum is everybody's neighbour there is one group.
+// (2048^2 white noise in 16 pieces, all levels: 12.4 ms as one group per merge,
+// 3.0 ms so, finding the groups included; a smooth 1025x769 field, one group: the
+// search costs 0.1 ms a level of 4.)
+//
+// A block takes a group at a time.  Its first warp walks the group's cells in the
+// loop's order, 32 at a time: their lanes look the
 // cells up side by side (cell -> point -> flags and pair -> the pair's cell)
 // and drop those the loop would skip whatever happens before their turn; then
 // the cells left are done one after the other (warp_graph.cuh).  A
@@ -630,7 +641,8 @@ struct SeqShared {
   TeamState team;
   WarpGraph::Pair pair;
   int stop;
-  long long at;  // first cell of the batch the first warp is at
+  long long at;    // the first warp's batch, as a place in the group
+  uint32_t first;  // the group's first place, NO_CP: none left
   uint2 stage[SEQ_WARPS * SEQ_STAGE];
 };
 __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
@@ -685,91 +697,217 @@ __device__ __forceinline__ int up_cell(const MGraph &M, const CRect &ixn, long l
 }
 __device__ __forceinline__ void seq_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * SEQ_WARPS) : "memory"); }
 
-__global__ void __launch_bounds__(32 * (SEQ_WARPS + 1)) k_merge_up_seq(MGraph *graphs, const SeqJob *jobs, int njobs, uint32_t *status) {
-  __shared__ SeqShared sh;
-  const int b = blockIdx.x;
-  if (b >= njobs) return;
-  const SeqJob jb = jobs[b];
-  const MGraph M = graphs[jb.g0];  // (a copy of the descriptor: pointers stay in registers)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long w = jb.ixn.r - jb.ixn.l + 1, n = w * (jb.ixn.t - jb.ixn.b + 1);
-  if (threadIdx.x == 0) {
-    sh.team.top = M.G.L.top;
-    sh.team.fail = 0;
-    sh.stop = 0;
-    sh.at = 0;
+// The groups of a job's boundary cells: cells [base, base + n) of the arrays
+// that all jobs share.
+struct UpWork {
+  uint32_t *slot;           // per critical point: the first cell that has it in its reach (null: no groups)
+  unsigned long long *top;  // the list pool's top
+  uint32_t *ctr;            // [0] groups, [1] groups taken, [2] 1: no groups, all cells in order, [3] blocks done
+  uint32_t base, n;
+};
+struct UpGroups {
+  const UpWork *work;
+  uint32_t *parent;       // union-find over a job's cells; NO_CP: the cell never acts
+  uint32_t *key, *cell;   // a place's group (its first cell, over all jobs) and cell, sorted by group; key = total: never acts
+  uint32_t *first;        // per job from base on: the groups' first places, in no order
+  uint32_t total;
+};
+constexpr int UP_BLOCKS = 64;  // blocks per job
+
+// The root of cell a; every step leaves a shortcut.  Parents only get smaller.
+__device__ __forceinline__ uint32_t group_of(uint32_t *parent, uint32_t a) {
+  volatile uint32_t *const p = parent;
+  for (;;) {  // (a falls with every step)
+    const uint32_t b = p[a];
+    if (b >= a) return a;
+    const uint32_t c = p[b];
+    if (c < b) p[a] = c;
+    a = b;
   }
-  __syncthreads();
-  if (warp == SEQ_WARPS) {  // reads ahead: at most one batch beyond the first warp's
-    for (long long t0 = 0; t0 < n; t0 += 32) {
-      for (long long polls = 0; *(volatile long long *)&sh.at + 32 < t0 && !*(volatile int *)&sh.stop && polls < (1ll << 26); ++polls) __nanosleep(200);
-      if (*(volatile int *)&sh.stop) break;
-      uint32_t si = 0, pi = 0;
-      if (t0 + lane < n && up_cell(M, jb.ixn, w, t0 + lane, si, pi) == 1) {
-        warm_point(M, si);
-        warm_point(M, pi);
+}
+__device__ __forceinline__ bool join_groups(uint32_t *parent, uint32_t a, uint32_t b) {
+  for (int guard = 0; guard < 1 << 20; ++guard) {  // (a failed CAS: the other thread's succeeded)
+    a = group_of(parent, a);
+    b = group_of(parent, b);
+    if (a == b) return true;
+    if (a > b) { const uint32_t c = a; a = b; b = c; }
+    if (atomicCAS(&parent[b], b, a) == b) return true;
+  }
+  return false;
+}
+__global__ void k_up_init(const MGraph *graphs, const SeqJob *jobs, UpGroups g) {
+  const UpWork w = g.work[blockIdx.y];
+  GRID_LOOP(t, (long long)w.n) g.parent[w.base + t] = (uint32_t)t;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *w.top = graphs[jobs[blockIdx.y].g0].G.L.top;
+    if (!w.slot) w.ctr[2] = 1;
+  }
+}
+// A warp per cell: a cell that may act leaves its number at its reach and is
+// joined with the cells that were there, one of each of their groups (32 cells a
+// warp and a join per point took 320 us on a smooth field's 2049 cells).
+__global__ void k_up_join(const MGraph *graphs, const SeqJob *jobs, UpGroups g) {
+  const UpWork wk = g.work[blockIdx.y];
+  const SeqJob jb = jobs[blockIdx.y];
+  const MGraph &M = graphs[jb.g0];
+  const int lane = threadIdx.x & 31;
+  const long long w = jb.ixn.r - jb.ixn.l + 1;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  uint32_t *const parent = g.parent + wk.base;
+  bool lost = false;
+  for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < wk.n; t += warps) {
+    uint32_t c[2] = {0, 0};
+    const int what = up_cell(M, jb.ixn, w, t, c[0], c[1]);
+    if (what > 1) lost = true;  // an error at its turn: the plain order
+    if (what == 0) parent[t] = NO_CP;
+    if (what != 1) continue;
+    auto reach = [&](bool on, uint32_t v) {
+      uint32_t old = t;
+      if (on && v < M.G.ncp) {
+        const uint32_t o = atomicMin(&wk.slot[v], t);
+        if (o != NO_CP) old = o;
       }
-      __syncwarp();
+      for (int guard = 0;; ++guard) {
+        const uint32_t r = group_of(parent, old), own = group_of(parent, t);
+        const unsigned apart = __ballot_sync(FULL_WARP, r != own);
+        if (!apart) break;
+        if (guard == 4096) { lost = true; break; }  // (others' joins may show roots apart that are not)
+        if (lane == __ffs(apart) - 1 && !join_groups(parent, r, own)) lost = true;
+        __syncwarp();
+      }
+    };
+    reach(lane < 2, c[lane & 1]);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const uint32_t q = 2 * c[l >> 1] + (l & 1), m = M.G.L.nrun[q];
+      const uint2 *r = M.G.L.pool + M.G.L.off[q];
+      for (uint32_t k0 = 0; k0 < m; k0 += 32) reach(k0 + lane < m, k0 + lane < m ? r[k0 + lane].x : 0);
     }
-    return;
   }
+  if (lost) wk.ctr[2] = 1;
+}
+__global__ void k_up_key(UpGroups g) {
+  const UpWork w = g.work[blockIdx.y];
+  GRID_LOOP(t, (long long)w.n) {
+    g.key[w.base + t] = g.parent[w.base + t] == NO_CP ? g.total : w.base + group_of(g.parent + w.base, (uint32_t)t);
+    g.cell[w.base + t] = (uint32_t)t;
+  }
+}
+__global__ void k_up_first(UpGroups g, int njobs) {
+  GRID_LOOP(q, (long long)g.total) {
+    const uint32_t k = g.key[q];
+    if (k >= g.total || (q > 0 && g.key[q - 1] == k)) continue;
+    int b = 0;
+    while (b + 1 < njobs && g.work[b + 1].base <= k) ++b;
+    g.first[g.work[b].base + atomicAdd(g.work[b].ctr, 1u)] = (uint32_t)q;
+  }
+}
+
+__global__ void __launch_bounds__(32 * (SEQ_WARPS + 1), 1) k_merge_up_seq(MGraph *graphs, const SeqJob *jobs, UpGroups g, uint32_t *status) {
+  __shared__ SeqShared sh;
+  const SeqJob jb = jobs[blockIdx.y];
+  const UpWork wk = g.work[blockIdx.y];
+  const bool plain = wk.ctr[2] != 0;  // all cells in order, by the job's first block
+  const MGraph M = graphs[jb.g0];     // (a copy of the descriptor: pointers stay in registers)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long w = jb.ixn.r - jb.ixn.l + 1;
   WarpGraph W;
   W.G = M.G;
   W.lane = lane;
   W.team = &sh.team;
-  W.stage = sh.stage + warp * SEQ_STAGE;
+  W.stage = sh.stage + (warp % SEQ_WARPS) * SEQ_STAGE;
   W.nstage = SEQ_STAGE;
-  W.G.tmp_cap = M.G.tmp_cap / SEQ_WARPS;
-  W.G.tmp = M.G.tmp + warp * W.G.tmp_cap;
-  if (warp > 0) {
-    for (;;) {
-      seq_barrier();
-      if (sh.stop) return;
-      W.edit_neighbours(sh.pair, warp, SEQ_WARPS);
-      if (W.G.fail) sh.team.fail = 1;
-      seq_barrier();
-    }
+  W.G.tmp_cap = M.G.tmp_cap / (SEQ_WARPS * gridDim.x);
+  W.G.tmp = M.G.tmp + (blockIdx.x * SEQ_WARPS + warp % SEQ_WARPS) * W.G.tmp_cap;
+  if (threadIdx.x == 0) {
+    sh.team.shared_top = wk.top;
+    sh.team.fail = 0;
+    sh.stop = 0;
   }
-  bool stop = false;
-  for (long long t0 = 0; t0 < n && !stop; t0 += 32) {
-    if (lane == 0) *(volatile long long *)&sh.at = t0;
-    uint32_t si = 0, pi = 0;
-    const int todo = t0 + lane < n ? up_cell(M, jb.ixn, w, t0 + lane, si, pi) : 0;
-    __syncwarp();
-    for (unsigned left = __ballot_sync(FULL_WARP, todo != 0); left && !stop; left &= left - 1) {
-      const int s = __ffs(left) - 1;
-      const int what = __shfl_sync(FULL_WARP, todo, s);
-      const uint32_t c = __shfl_sync(FULL_WARP, si, s), d = __shfl_sync(FULL_WARP, pi, s);
-      if (what != 2 && (M.G.flags[c] & F_CANCELLED)) continue;  // with an earlier cell
-      if (what != 1) {  // "missing common bndry cp", or a partner outside the complex
-        if (lane == 0) set_status(status, ST_INVARIANT);
-        stop = true;
-        break;
+  for (bool more = !plain || blockIdx.x == 0; more;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      sh.at = 0;
+      sh.first = 0;
+      if (!plain && !sh.team.fail) {
+        const uint32_t q = atomicAdd(wk.ctr + 1, 1u);
+        sh.first = q < wk.ctr[0] ? g.first[wk.base + q] : NO_CP;
       }
-      WarpGraph::Pair q{reinterpret_cast<const uint2 *>(M.G.L.off)[c], reinterpret_cast<const uint2 *>(M.G.L.off)[d],
-                        reinterpret_cast<const uint2 *>(M.G.L.nrun)[c], reinterpret_cast<const uint2 *>(M.G.L.nrun)[d], c, d};
-      if (!W.orient(q)) continue;
-      if (lane == 0) sh.pair = q;
-      seq_barrier();
-      W.edit_neighbours(q, 0, SEQ_WARPS);
-      if (W.G.fail) sh.team.fail = 1;
-      seq_barrier();
-      W.close(q, 0);
-      __syncwarp();
-      if (sh.team.fail) stop = true;
+      if (sh.team.fail || sh.stop == 2) sh.first = NO_CP;
+      sh.stop = 0;
     }
+    __syncthreads();
+    const uint32_t first = sh.first, key = plain || first == NO_CP ? 0 : g.key[first];
+    if (first == NO_CP) break;
+    more = !plain;
+    // the group's cell at place k, -1 past its end
+    auto cell_at = [&](long long k) -> long long {
+      if (plain) return k < wk.n ? k : -1;
+      return first + k < g.total && g.key[first + k] == key ? (long long)g.cell[first + k] : -1;
+    };
+    if (warp == SEQ_WARPS) {  // reads ahead: at most one batch beyond the first warp's
+      for (long long t0 = 0;; t0 += 32) {
+        const long long t = cell_at(t0 + lane);
+        if (!__any_sync(FULL_WARP, t >= 0)) break;
+        for (long long polls = 0; *(volatile long long *)&sh.at + 32 < t0 && !*(volatile int *)&sh.stop && polls < (1ll << 26); ++polls) __nanosleep(200);
+        if (__any_sync(FULL_WARP, *(volatile int *)&sh.stop)) break;
+        uint32_t si = 0, pi = 0;
+        if (t >= 0 && up_cell(M, jb.ixn, w, t, si, pi) == 1) {
+          warm_point(M, si);
+          warm_point(M, pi);
+        }
+        __syncwarp();
+      }
+      continue;
+    }
+    if (warp > 0) {
+      for (;;) {
+        seq_barrier();
+        if (sh.stop) break;
+        if (warp == SEQ_WARPS - 1) W.close(sh.pair, 0);  // (nobody reads what it changes until the next pair)
+        W.edit_neighbours(sh.pair, warp, SEQ_WARPS);
+        if (W.G.fail) sh.team.fail = 1;
+        seq_barrier();
+      }
+      continue;
+    }
+    int stop = 0;
+    for (long long t0 = 0; !stop; t0 += 32) {
+      if (lane == 0) *(volatile long long *)&sh.at = t0;
+      uint32_t si = 0, pi = 0;
+      const long long t = cell_at(t0 + lane);
+      if (!__any_sync(FULL_WARP, t >= 0)) break;
+      const int todo = t >= 0 ? up_cell(M, jb.ixn, w, t, si, pi) : 0;
+      __syncwarp();
+      for (unsigned left = __ballot_sync(FULL_WARP, todo != 0); left && !stop; left &= left - 1) {
+        const int s = __ffs(left) - 1;
+        const int what = __shfl_sync(FULL_WARP, todo, s);
+        const uint32_t c = __shfl_sync(FULL_WARP, si, s), d = __shfl_sync(FULL_WARP, pi, s);
+        if (what != 2 && (M.G.flags[c] & F_CANCELLED)) continue;  // with an earlier cell
+        if (what != 1) {  // "missing common bndry cp", or a partner outside the complex
+          if (lane == 0) set_status(status, ST_INVARIANT);
+          stop = 2;
+          break;
+        }
+        WarpGraph::Pair q{reinterpret_cast<const uint2 *>(M.G.L.off)[c], reinterpret_cast<const uint2 *>(M.G.L.off)[d],
+                          reinterpret_cast<const uint2 *>(M.G.L.nrun)[c], reinterpret_cast<const uint2 *>(M.G.L.nrun)[d], c, d};
+        if (!W.orient(q)) continue;
+        if (lane == 0) sh.pair = q;
+        seq_barrier();
+        W.edit_neighbours(q, 0, SEQ_WARPS);
+        if (W.G.fail) sh.team.fail = 1;
+        seq_barrier();
+        if (sh.team.fail) stop = 2;
+      }
+    }
+    if (lane == 0) *(volatile int *)&sh.stop = stop ? stop : 1;
+    __syncwarp();
+    seq_barrier();
   }
-  if (lane == 0) {
-    *(volatile int *)&sh.stop = 1;
-    MGraph g = M;
-    g.G.fail = sh.team.fail != 0;
-    g.G.ops = W.G.ops;
-    g.G.L.top = sh.team.top;
-    if (g.G.fail) set_status(status, ST_SIMPLIFY_LIMIT);
-    graphs[jb.g0] = g;
-  }
-  __syncwarp();
-  seq_barrier();
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (sh.team.fail) set_status(status, ST_SIMPLIFY_LIMIT);
+  if (atomicAdd(wk.ctr + 3, 1u) + 1 == gridDim.x) graphs[jb.g0].G.L.top = atomicAdd(wk.top, 0ull);
 }
 
 // merge_down's boundary uncancellations, one job per block.  The loop runs in
@@ -816,6 +954,7 @@ __global__ void __launch_bounds__(32 * DOWN_WARPS, 1) k_merge_down_seq(MGraph *g
   const long long w = jb.ixn.r - jb.ixn.l + 1, n = w * (jb.ixn.t - jb.ixn.b + 1);
   if (threadIdx.x == 0) {
     team.top = M.G.L.top;
+    team.shared_top = nullptr;
     team.fail = team.wrong = 0;
     team.lock = 0;
     odd = n > DOWN_CELLS;
@@ -1164,9 +1303,29 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
     poff[k] = sbytes;
     sbytes += sizeof(uint2) * ((size_t)(x.r - x.l + 1) * (x.t - x.b + 1) + 15) / 16 * 16;
   }
+  // merge_up's jobs in groups: per job a slot per critical point; over all jobs
+  // six words per boundary cell; a pool top and four counters per job
+  const bool groups = !down && !rounds;
+  size_t slot_bytes = 0, cells = 0;
+  std::vector<size_t> base(nj, 0);
+  for (size_t k = 0; k < nj && groups; ++k) {
+    const CRect &x = jobs[k].ixn;
+    soff[k] = slot_bytes;
+    base[k] = cells;
+    slot_bytes += 4ull * ((mg(*graphs[jobs[k].g0]).G.ncp + 1 + 31) / 32 * 32);
+    cells += (size_t)(x.r - x.l + 1) * (x.t - x.b + 1);
+  }
+  const size_t cell_bytes = (24 * cells + 15) / 16 * 16;
+  if (groups) sbytes = cell_bytes + 32 * nj + slot_bytes;
   const size_t head = (gb + 15) / 16 * 16 + (jbytes + 15) / 16 * 16;
-  const size_t pbytes = ((rounds ? 8ull : down ? sizeof(DownWork) : 0ull) * nj + 15) / 16 * 16;
+  const size_t pbytes = ((rounds ? 8ull : down ? sizeof(DownWork) : sizeof(UpWork)) * nj + 15) / 16 * 16;
   cudaError_t e = cudaMallocAsync((void **)&buf, head + pbytes + sbytes + 64, st);
+  if (e == cudaErrorMemoryAllocation && groups) {  // no room for the slots: all cells in order
+    cudaGetLastError();
+    sbytes -= slot_bytes;
+    slot_bytes = 0;
+    e = cudaMallocAsync((void **)&buf, head + pbytes + sbytes + 64, st);
+  }
   if (e != cudaSuccess) return e;
   MGraph *dg = (MGraph *)buf;
   SeqJob *dj = (SeqJob *)(buf + ((gb + 15) / 16) * 16);
@@ -1191,6 +1350,21 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
     if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, obytes, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // hw is read before it goes out of scope
   }
+  UpGroups ug{};
+  if (e == cudaSuccess && groups) {
+    char *const words = buf + head + pbytes, *const ctr = words + cell_bytes, *const slot = ctr + 32 * nj;
+    uint32_t *const at = (uint32_t *)words;
+    ug = UpGroups{(const UpWork *)(buf + head), at, at + cells, at + 2 * cells, at + 3 * cells, (uint32_t)cells};
+    std::vector<UpWork> hw(nj);
+    for (size_t k = 0; k < nj; ++k)
+      hw[k] = UpWork{slot_bytes ? (uint32_t *)(slot + soff[k]) : nullptr, (unsigned long long *)(ctr + 32 * k),
+                     (uint32_t *)(ctr + 32 * k + 8), (uint32_t)base[k],
+                     (uint32_t)((k + 1 < nj ? base[k + 1] : cells) - base[k])};
+    e = cudaMemcpyAsync(buf + head, hw.data(), sizeof(UpWork) * nj, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctr, 0, 32 * nj, st);
+    if (e == cudaSuccess && slot_bytes) e = cudaMemsetAsync(slot, 0xFF, slot_bytes, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // hw is read before it goes out of scope
+  }
   if (e == cudaSuccess) {
     k_seq_prefetch<<<dim3(64, (unsigned)nj), 256, 0, st>>>(dg, dj, nullptr);
     if (rounds) {
@@ -1206,7 +1380,20 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
       if (e == cudaSuccess)
         k_merge_down_seq<<<(unsigned)nj, 32 * DOWN_WARPS, DOWN_SMEM, st>>>(dg, dj, (int)nj, (const DownWork *)(buf + head), status);
     } else {
-      k_merge_up_seq<<<(unsigned)nj, 32 * (SEQ_WARPS + 1), 0, st>>>(dg, dj, (int)nj, status);
+      const dim3 grid(32, (unsigned)nj);
+      k_up_init<<<grid, 256, 0, st>>>(dg, dj, ug);
+      DMSC_LAUNCHED(1);
+      if (slot_bytes) {
+        k_up_join<<<dim3(256, (unsigned)nj), 256, 0, st>>>(dg, dj, ug);
+        k_up_key<<<grid, 256, 0, st>>>(ug);
+        int bits = 1;
+        while (bits < 32 && (ug.total >> bits)) ++bits;
+        e = radix_sort_pairs(ug.key, ug.cell, ug.first + cells, ug.first + 2 * cells, (long long)cells, bits, st);
+        k_up_first<<<64, 256, 0, st>>>(ug, (int)nj);
+        DMSC_LAUNCHED(3);
+      }
+      if (e == cudaSuccess)
+        k_merge_up_seq<<<dim3(slot_bytes ? UP_BLOCKS : 1, (unsigned)nj), 32 * (SEQ_WARPS + 1), 0, st>>>(dg, dj, ug, status);
     }
     DMSC_LAUNCHED(2);
     if (e == cudaSuccess) e = cudaGetLastError();

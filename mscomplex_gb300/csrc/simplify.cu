@@ -655,6 +655,7 @@ __global__ void __launch_bounds__(32 * SIMP_WARPS, 2) k_simplify(SimpArgs *args,
   const SimpArgs a = args[blockIdx.x];
   if (threadIdx.x == 0) {
     sh.team.top = a.G.L.top;
+    sh.team.shared_top = nullptr;
     sh.team.ops = 0;
     sh.team.fail = sh.team.wrong = 0;
     sh.stop = 0;
@@ -712,6 +713,7 @@ __global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, ui
   W.done = words <= DONE_WORDS ? reinterpret_cast<uint32_t *>(W.shared_stage + shared_runs) : reinterpret_cast<uint32_t *>(a.resub);
   if (threadIdx.x == 0) {
     team.top = a.G.L.top;
+    team.shared_top = nullptr;
     team.ops = a.G.ops;
     team.ticket = 2ull * a.ncanc;
     team.fail = team.wrong = 0;

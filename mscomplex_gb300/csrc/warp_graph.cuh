@@ -46,6 +46,7 @@ struct TeamState {
   unsigned long long ticket; // pairs not yet taken
   uint32_t fail, wrong;      // a pool, budget or wait ran out; a reference logic_error condition
   int lock;                  // 1: a warp uses the scratch all warps share
+  unsigned long long *shared_top;  // the pool's top where several blocks edit the graph (then top is unused)
 };
 constexpr unsigned long long WAIT_LIMIT = 1ull << 26;  // polls of a wait on another warp
 constexpr int BAR_EDIT = 3;
@@ -598,11 +599,11 @@ struct WarpGraph {
     if (lane == 0) { G.L.off[l] = off; G.L.cap[l] = nc; }
     return true;
   }
-  // n runs at the top of the pool (shared by the team's warps)
+  // n runs at the top of the pool (shared by the team's warps, or by all blocks)
   __device__ __forceinline__ unsigned long long take_room(unsigned long long n) {
     unsigned long long at = G.L.top;
     if (team) {
-      if (lane == 0) at = atomicAdd(&team->top, n);
+      if (lane == 0) at = team->shared_top ? atomicAdd(team->shared_top, n) : atomicAdd(&team->top, n);
       at = __shfl_sync(FULL_WARP, at, 0);
     }
     if (at + n > G.L.pool_cap) G.fail = true;
