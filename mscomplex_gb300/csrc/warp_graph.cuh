@@ -158,12 +158,97 @@ struct WarpGraph {
         return;
       }
     }
+    // up to four values: eight runs a lane, all in flight at once, and each value's
+    // place from ballots (a list of 100 runs: 3300 cycles by the searches and
+    // moves below, 1000 so)
+    if (n <= 256 && sn <= 4) {
+      constexpr int K = 8;
+      uint2 v[K], s = make_uint2(skip, 0u);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        v[k] = make_uint2(0xffffffffu, 0u);
+        if (k * 32u + lane < n) v[k] = p[k * 32 + lane];
+      }
+      if ((uint32_t)lane < sn) s = S[lane];
+      uint32_t e = n, ey = 0;
+      if (has_r) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if (k * 32u >= n) break;
+          const unsigned b = __ballot_sync(FULL_WARP, v[k].x == r);
+          if (b) {
+            e = k * 32 + __ffs(b) - 1;
+            ey = __shfl_sync(FULL_WARP, v[k].y, __ffs(b) - 1);
+          }
+        }
+      }
+      const bool ex = e < n;
+      uint32_t at[4], fresh = 0, changed = 0, ebef = 0, pos = 0;  // places of the added runs (n: none there)
+      unsigned long long ticks = 0, add = 0;
+      bool bad = false;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        at[j] = 0xffffffffu;
+        if (j >= (int)sn) continue;
+        const uint32_t x = __shfl_sync(FULL_WARP, s.x, j);
+        if (x == skip) continue;
+        const unsigned long long c = (unsigned long long)__shfl_sync(FULL_WARP, s.y, j) * mult;
+        if (c > 0xffffffffull) bad = true;
+        uint32_t below = 0;
+        bool here = false;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if (k * 32u >= n) break;
+          below += __popc(__ballot_sync(FULL_WARP, v[k].x < x));
+          if (v[k].x == x) {
+            here = true;
+            if (v[k].y > 0xffffffffu - (uint32_t)c) bad = true;
+            v[k].y += (uint32_t)c;
+            changed |= 1u << k;
+          }
+        }
+        const bool dup = __any_sync(FULL_WARP, here);
+        if (!dup) {
+          at[j] = below;
+          fresh |= 1u << j;
+          ticks += n - below;
+          ebef += x < r ? 1u : 0u;
+          if (lane == j) pos = below;
+        }
+        add += c;
+        if (mark_a && lane == j && (dup || c >= 2)) mark(l >> 1, x);
+      }
+      if (mark_a) ticks += add;
+      const uint32_t knew = __popc(fresh), m = n + knew - (ex ? 1u : 0u);
+      if (ex) ticks += n + knew - (e + ebef);
+      if (__any_sync(FULL_WARP, bad) || tot + add > 0xffffffffull) { G.fail = true; return; }
+      uint32_t off = off0;
+      if (m > cap && !grow(l, cap, m, off)) return;
+      uint2 *const dst = G.L.pool + off;
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        if (k * 32u >= n) break;
+        const uint32_t i = k * 32 + lane;
+        const uint32_t to = i + (at[0] <= i) + (at[1] <= i) + (at[2] <= i) + (at[3] <= i) - (ex && i > e ? 1u : 0u);
+        if (i < n && i != e && (dst != p || to != i || (changed >> k & 1))) dst[to] = v[k];
+      }
+      if (fresh >> lane & 1)
+        dst[pos + __popc(fresh & lt()) - (ex && e < pos ? 1u : 0u)] = make_uint2(s.x, (uint32_t)((unsigned long long)s.y * mult));
+      if (lane == 0) { G.L.nrun[l] = m; G.L.total[l] = tot + (uint32_t)add - ey; }
+      __syncwarp();
+      G.tick(ticks);
+      return;
+    }
     // the values and the added runs (value, count; place, 0) in shared memory
     // where they fit: the searches below are chains of dependent loads
     uint2 *fr = G.tmp;
     const uint32_t *X = &p[0].x;
     uint32_t xs = 2, e = 0;  // e: the removed run's index + 1
-    const bool staged = 2ull * sn + (n + 1) / 2 <= nstage;
+    // a few values: each by all lanes, 32 probes a round, without a look at all runs
+    const bool few = sn <= 4 && nstage >= 8;
+    const bool staged = !few && 2ull * sn + (n + 1) / 2 <= nstage;
+    if (few) fr = stage;
     if (staged) {
       fr = stage;
       uint32_t *sx = reinterpret_cast<uint32_t *>(stage + 2 * sn);
@@ -178,7 +263,7 @@ struct WarpGraph {
       e = __reduce_max_sync(FULL_WARP, e);
       __syncwarp();
     } else {
-      if (2ull * sn > G.tmp_cap) { G.fail = true; return; }
+      if (!few && 2ull * sn > G.tmp_cap) { G.fail = true; return; }
       if (has_r) {
         e = lower(p, n, r);
         e = e < n && p[e].x == r ? e + 1 : 0;
@@ -206,9 +291,14 @@ struct WarpGraph {
       const unsigned long long c = (unsigned long long)s.y * mult;
       uint32_t pos = 0;
       bool dup = false;
+      if (few)
+        for (uint32_t j = 0; j < sn; ++j) {
+          const uint32_t at = lower(p, n, __shfl_sync(FULL_WARP, s.x, j));
+          if ((uint32_t)lane == j) pos = at;
+        }
       if (valid) {
         if (c > 0xffffffffull) bad = true;
-        pos = lower_x(s.x);
+        if (!few) pos = lower_x(s.x);
         dup = pos < n && X[pos * xs] == s.x;
         if (dup) {
           const uint32_t y = p[pos].y;
@@ -253,10 +343,12 @@ struct WarpGraph {
       }
       return lo;
     };
-    constexpr int U = 4;  // runs per lane in flight
+    constexpr int U = 8;  // runs per lane in flight
     const uint32_t first = dst == p ? min(pos0, e) : 0;  // runs before it keep their place
-    // runs that move to a higher place, from the back (in a new place: all runs)
-    for (uint32_t hi = n; hi > first;) {
+    // runs that move to a higher place, from the back (in a new place: all runs;
+    // with one added run for the removed one, those between the two places)
+    const uint32_t end = dst != p || knew > 1 || (knew == 1 && !ex) ? n : knew == 1 && pos0 <= e ? e : first;
+    for (uint32_t hi = end; hi > first;) {
       const uint32_t lo = hi - first > 32 * U ? hi - 32 * U : first;
       uint2 v[U];
       uint32_t to[U];
@@ -435,7 +527,7 @@ struct WarpGraph {
     const uint2 *pA = G.L.pool + o0.x, *pD = G.L.pool + o1.y;
     const uint32_t nA = q.n0.x, nE0 = q.n0.y, nE1 = q.n1.x, nD = q.n1.y;
     const uint32_t tD = nA, tE0 = nA + nD, tE1 = tE0 + nE0, nt = tE1 + nE1;
-    int turn = 0;  // the warp that takes the next longer list
+    int turn = 0;  // the warp that took the last longer list
     // The added value of either side where there is at most one (k: how many, 2
     // for more): the list without the other point, from its first two runs.
     uint2 fA[2], fD[2];
@@ -467,18 +559,24 @@ struct WarpGraph {
         asm volatile("bar.sync %0, %1;" ::"r"(BAR_EDIT), "r"(32 * warps) : "memory");
       }
       if (G.fail) continue;
-      // the longer lists' lines on their way into L1
-      if (side >= 0 && !small)
-        for (uint32_t q = 0; q < n && q < 256; q += 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(G.L.pool + off + q));
+      // the long lists' first lines on their way into L1
+      if (side >= 0 && n > 256)
+        for (uint32_t q = 0; q < 256; q += 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(G.L.pool + off + q));
       // (mostly a saddle's neighbours or an extremum's saddles: two runs, one added value)
       if (who == 0) {
         if (!__any_sync(FULL_WARP, small && n > 4)) lane_edits<4>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0);
         else lane_edits<8>(small, l, n, cap, tot, off, ad, ka, mult, r, side == 0);
       }
-      // the longer lists, each by all lanes of a warp
-      for (unsigned big = __ballot_sync(FULL_WARP, side >= 0 && !small); big && !G.fail; big &= big - 1) {
-        turn = turn + 1 == warps ? 0 : turn + 1;  // (warp 0 last: it has the short lists)
-        if (turn != who) continue;
+      // the longer lists, each by all lanes of a warp; they go round from the warp
+      // after the last one that took one (warp 0 last: it has the short lists)
+      unsigned big = __ballot_sync(FULL_WARP, side >= 0 && !small);
+      const int nbig = __popc(big);
+      int wait = (who + 2 * warps - turn - 1) % warps;  // lists before this warp's first
+      turn = (turn + nbig) % warps;
+      if (wait >= nbig) continue;
+      for (; big && !G.fail; big &= big - 1) {
+        if (wait-- != 0) continue;
+        wait = warps - 1;
         const int s = __ffs(big) - 1;
         const int bs = __shfl_sync(FULL_WARP, side, s);
         const uint32_t bl = __shfl_sync(FULL_WARP, l, s), bm = __shfl_sync(FULL_WARP, mult, s);
