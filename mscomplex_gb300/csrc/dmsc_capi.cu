@@ -184,7 +184,7 @@ static int dataset_work(dmsc_dataset *d, void *stream, int desc) {
     CK(cudaMemsetAsync(d->cp_acnt.p, 0, sizeof(uint32_t) * d->cap, st));
     CK(cudaMemsetAsync(d->cp_dcnt.p, 0, sizeof(uint32_t) * d->cap, st));
     CpOut cp{d->cp_cellid.p, d->cp_fn.p, d->cp_flags.p, d->cp_pair_cell.p, d->cp_des2.p,
-             d->cp_asc2.p, d->cp_acnt.p, d->cp_dcnt.p, d->cap};
+             d->cp_asc2.p, d->cp_acnt.p, d->cp_dcnt.p, d->cap, d->scal.p + 1};
     if (tm) CK(cudaEventRecord(d->ev[3], st));
     CK(launch_labels(d->codes.p, d->terms.p, d->hgt, g, d->offsets.p, d->table.p, d->labels.p, cp, d->scal.p, st));
     if (tm) CK(cudaEventRecord(d->ev[4], st));

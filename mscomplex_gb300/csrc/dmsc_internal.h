@@ -22,6 +22,7 @@ struct CpOut {
   uint32_t *acnt;     // per cp: |asc| (saddles written, minima counted atomically)
   uint32_t *dcnt;     // per cp: |des|
   long long cap;      // capacity of every array above (in critical points)
+  const uint32_t *count = nullptr;  // how many there will be, if not known to fit
 };
 
 // One grid of a batch: its geometry (with batch-wide slot / segment bases)

@@ -576,6 +576,12 @@ __device__ __forceinline__ void labels_tile_t(const uint32_t *__restrict__ codes
   uint32_t *const labV = &s.labV[0][0], *const labF = &s.labF[1][1];  // entry (i, j) at j * LS + i
   constexpr int LS = TX + 1;
 
+  // arrays too small for the critical points: nothing is done (the caller grows
+  // them and calls again; 4096x4096 quantised heights: 0.15 ms of labels saved)
+  if (cp.count && *cp.count > cp.cap) {
+    if (threadIdx.x == 0) atomicOr(status, ST_CAPACITY);
+    return;
+  }
   uint32_t code[ROWS], term[ROWS];
   const long long at0 = (long long)(ty0 + j0) * g.vnx + tx0 + i;
 #pragma unroll
