@@ -17,8 +17,9 @@
 //     uncancelled points -- counts, a scan, a scatter, and a sort of each list
 //     by index (the ascending order in which a std::multiset iterates);
 //   * the cancellations along the shared boundary (:124-153), row-major and
-//     order dependent: one block per merge, on the mutable graph
-//     (k_merge_up_seq), all merges of the level in one launch.
+//     order dependent among cells that touch a common point: on the mutable
+//     graph, one block per group of such cells (k_merge_up_seq), all merges of
+//     the level in one launch.
 // merge_down (:158-322) splits into
 //   * the uncancellations along the shared boundary (:172-201): one block per
 //     parent (k_merge_down_seq), all merges of the level in one launch;
@@ -797,8 +798,11 @@ __global__ void k_up_first(UpGroups g, int njobs) {
   GRID_LOOP(q, (long long)g.total) {
     const uint32_t k = g.key[q];
     if (k >= g.total || (q > 0 && g.key[q - 1] == k)) continue;
-    int b = 0;
-    while (b + 1 < njobs && g.work[b + 1].base <= k) ++b;
+    int b = 0;  // the last job that starts at or before cell k
+    for (int hi = njobs - 1; b < hi;) {
+      const int m = (b + hi + 1) >> 1;
+      if (g.work[m].base <= k) b = m; else hi = m - 1;
+    }
     g.first[g.work[b].base + atomicAdd(g.work[b].ctr, 1u)] = (uint32_t)q;
   }
 }

@@ -38,3 +38,23 @@ def test_groups(gpu_lib, oracle, kind, ny, nx, levels, split2d):
         assert_same_complex(got.piece(i).export(), want.piece(i), f"{kind} {nx}x{ny} node {i}", keys=GRAPH)
     del got
     ctx.close()
+
+
+@pytest.mark.parametrize("up", [True, False])
+@pytest.mark.parametrize("n", [301, 421])
+def test_a_boundary_point_with_thousands_of_saddles(gpu_lib, oracle, n, up):
+    """A funnel of peaks drains to one point of the shared boundary, which pairs
+    across it: cancelling it moves more values than a warp's scratch holds."""
+    y, x = np.mgrid[0:n, 0:n].astype(np.float64)
+    row = n // 2
+    far = np.hypot(x - n // 2, y - row)
+    side = y >= row if up else y <= row
+    f = np.where(side, far, -far - 1.0)
+    f[row, :] = far[row, :]
+    f[side & (y % 3 == 0) & (x % 3 == 1) & (np.abs(y - row) > 1)] += 9.0
+    f = f.astype(np.float32)
+    want = oracle.Pipeline(f, levels=1, tresh=0.0, split2d=False)
+    assert np.diff(want.piece(2)["asc_off"]).max() > 5000
+    got = gpu_lib.GridDataManager(f, levels=1, tresh=0.0, split2d=False)
+    for i in range(3):
+        assert_same_complex(got.piece(i).export(), want.piece(i), f"funnel {n} node {i}", keys=GRAPH)
