@@ -74,7 +74,7 @@ struct dmsc_pipeline {
   DevBuf<float> field;                    // device copy when the input was on the host
   DevBuf<uint32_t> status;
   double ms[5] = {0, 0, 0, 0, 0};
-  double seq_ms[2] = {0, 0};  // one-thread steps of the parallel merges: up, down
+  double seq_ms[2] = {0, 0};  // boundary steps of the parallel merges: up, down
   unsigned long long simp[5] = {0, 0, 0, 0, 0};
   // out of core (GridDataManager's compute_out_of_core): the archive file
   // prefix of this run, and per tree node whether its archive exists

@@ -61,7 +61,8 @@ class Context:
 
     def set_merge_rounds(self, window: int = 0, min_commits: int = 4):
         """merge_up's boundary cancellations on the parallel merges: 0 (the
-        default) runs them on one thread per merge; window > 0 in rounds over
+        default) runs them in groups that touch no common point, a block per
+        group; window > 0 in rounds over
         the first `window` pending boundary cells, one thread finishing in
         order after 8 rounds in a row below `min_commits` commits.  Every
         setting gives the same complexes."""
@@ -371,8 +372,7 @@ class GridDataManager:
 
     def merge_seq_times(self) -> dict:
         """Of merge up / down, the ms spent in the boundary steps (merge up's
-        cancellations in ordered-parallel rounds, merge down's uncancellations
-        on one thread per merge)."""
+        cancellations, merge down's uncancellations)."""
         ms = np.zeros(2, np.float64)
         check(self.lib.dmsc_pipeline_merge_times(self.h, _ptr(ms)))
         return {"merge_up": float(ms[0]), "merge_down": float(ms[1])}
