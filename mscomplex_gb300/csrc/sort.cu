@@ -8,11 +8,15 @@
 // that already run), groups the tile by digit in shared memory, and writes
 // every group as one contiguous piece.  Memory bounds it, 16 bytes a pair and
 // pass, and with it the look-back, whose traffic goes with the square of the
-// tiles in flight (256 words for each tile before a tile): a tile is as large
-// as one block's registers and shared memory allow, one block per SM.  With
-// 6,144 pairs a tile a pass over 3,000,017 took 41 us, with 20,480 31; a
+// tiles in flight (256 words for each tile before a tile): for many pairs a tile
+// is as large as one block's registers and shared memory allow, one block per SM.
+// With 6,144 pairs a tile a pass over 3,000,017 took 41 us, with 20,480 31; a
 // histogram, a scan and a scatter of single pairs took 77 (a warp's 32 pairs
-// went to 32 places).  Up to one tile is sorted by one block in one launch.
+// went to 32 places).  Such tiles leave SMs idle and are long for fewer pairs: up to
+// 1.6 million the tiles have 4,096 (a call with 130,000 pairs 158 us with 20,480 a
+// tile, 90 so; 900,000: 165, 125; 1,500,000: 169, 154).  Up to 8,192 pairs are
+// sorted by one block in one launch, 4 or 8 a thread (a call with 3,000 pairs 104
+// us with 20 a thread, 51 so; 6,000: 104, 61).
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 
@@ -22,21 +26,29 @@ namespace dmsc {
 
 namespace {
 
-constexpr int RS_THREADS = 1024, RS_WARPS = RS_THREADS / 32, RS_ITEMS = 20;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;  // each warp owns a contiguous run of 32 * RS_ITEMS pairs
+constexpr int RS_THREADS = 1024, RS_WARPS = RS_THREADS / 32;
+// pairs per thread; each warp owns a contiguous run of 32 times as many, a tile
+// has RS_THREADS times as many
+constexpr int RS_ITEMS = 20, RS_FEW = 4, RS_SMALL = 8;
+constexpr long long RS_FEW_MAX = 400ll * RS_THREADS * RS_FEW;
+// pairs of the tiles that n pairs are cut into (n of them: one launch)
+constexpr long long radix_tile(long long n) {
+  return RS_THREADS * (n <= RS_THREADS * RS_SMALL ? RS_SMALL : n <= RS_FEW_MAX ? RS_FEW : RS_ITEMS);
+}
 constexpr int RS_LOOK = 8;                      // earlier tiles looked at together
 constexpr int RS_MAX_PASSES = 8;                // 4 digits of the key, up to 4 of the array number
 constexpr unsigned long long RS_LIMIT = 1ull << 22;  // polls of an earlier tile's word
 
+template <int ITEMS>
 struct RadixSmem {
-  uint32_t key[RS_TILE], val[RS_TILE];
+  uint32_t key[RS_THREADS * ITEMS], val[RS_THREADS * ITEMS];
   uint16_t cnt[RS_WARPS][256];  // per warp and digit: pairs, then the pairs of the warps before it
   uint32_t first[256];          // the digit's first place in the tile
   uint32_t to[256];             // a pair's place in the output, less its place in the tile
   uint32_t wsum[8];
   uint32_t tile, late;
 };
-static_assert(RS_TILE < 65536, "places in a tile fit 16 bits");
+static_assert(RS_THREADS * RS_ITEMS < 65536, "places in a tile fit 16 bits");
 
 // One pass: digit = (key >> shift) & 255, or with len the digit of the value's
 // array number (value / len; the value is then the pair's original index).
@@ -56,17 +68,17 @@ __device__ __forceinline__ uint32_t digit_of(uint32_t key, uint32_t val, int shi
 // A tile's pairs: loaded, ranked by digit, and grouped in S.key / S.val in
 // stable order; S.first has each digit's first place.  Returns, for threads
 // below 256, the tile's pairs of digit threadIdx.x.
-template <bool ARRAY>
-__device__ __forceinline__ uint32_t group_tile(RadixSmem &S, const RadixPass &P, long long base0, long long n, bool from_smem) {
+template <bool ARRAY, int ITEMS>
+__device__ __forceinline__ uint32_t group_tile(RadixSmem<ITEMS> &S, const RadixPass &P, long long base0, long long n, bool from_smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   for (int k = threadIdx.x; k < RS_WARPS * 128; k += RS_THREADS) reinterpret_cast<uint32_t *>(&S.cnt[0][0])[k] = 0;
-  const long long base = base0 + warp * (32 * RS_ITEMS) + lane;
-  const int left = (int)(n - base < 32 * RS_ITEMS ? n - base : 32 * RS_ITEMS);  // pairs r * 32 < left are in range
-  uint32_t key[RS_ITEMS], val[RS_ITEMS];
-  uint16_t rank[RS_ITEMS];
+  const long long base = base0 + warp * (32 * ITEMS) + lane;
+  const int left = (int)(n - base < 32 * ITEMS ? n - base : 32 * ITEMS);  // pairs r * 32 < left are in range
+  uint32_t key[ITEMS], val[ITEMS];
+  uint16_t rank[ITEMS];
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     key[r] = val[r] = 0;
     if (r * 32 < left) {
       const long long i = base + r * 32;
@@ -81,7 +93,7 @@ __device__ __forceinline__ uint32_t group_tile(RadixSmem &S, const RadixPass &P,
   }
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     const bool valid = r * 32 < left;
     const uint32_t d = digit_of<ARRAY>(key[r], val[r], P.shift, P.len);
     uint32_t peers = __ballot_sync(0xffffffffu, valid);  // the lanes with the same digit
@@ -99,7 +111,7 @@ __device__ __forceinline__ uint32_t group_tile(RadixSmem &S, const RadixPass &P,
   }
   if (!ARRAY && !from_smem) {  // the values, while the digits are summed
 #pragma unroll
-    for (int r = 0; r < RS_ITEMS; ++r)
+    for (int r = 0; r < ITEMS; ++r)
       if (r * 32 < left) val[r] = P.vin ? P.vin[base + r * 32] : (uint32_t)(base + r * 32);
   }
   __syncthreads();
@@ -128,7 +140,7 @@ __device__ __forceinline__ uint32_t group_tile(RadixSmem &S, const RadixPass &P,
   }
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     if (r * 32 >= left) continue;
     const uint32_t d = digit_of<ARRAY>(key[r], val[r], P.shift, P.len), p = S.first[d] + S.cnt[warp][d] + rank[r];
     S.key[p] = key[r];
@@ -173,21 +185,22 @@ __global__ void __launch_bounds__(1024) k_radix_hist(const uint32_t *__restrict_
 // word[256 * tile + digit] of a pass: (flag in the top bits, pairs of the digit), flag
 // 0 not yet, 1 in the tile, 2 in the tile and all before it; W is 32 bits wide
 // below 2^30 pairs.
-template <bool ARRAY, typename W>
+template <bool ARRAY, typename W, int ITEMS>
 __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_pass(RadixPass P, long long n, const uint32_t *__restrict__ hist,
                                                               W *__restrict__ word, uint32_t *__restrict__ counter) {
   constexpr int FLAG = sizeof(W) == 4 ? 30 : 32;
   constexpr W COUNT = ((W)1 << FLAG) - 1;
   extern __shared__ __align__(16) unsigned char radix_smem[];
-  RadixSmem &S = *reinterpret_cast<RadixSmem *>(radix_smem);
+  constexpr int TILE = RS_THREADS * ITEMS;
+  RadixSmem<ITEMS> &S = *reinterpret_cast<RadixSmem<ITEMS> *>(radix_smem);
   if (threadIdx.x == 0) {
     S.tile = atomicAdd(counter, 1u);
     S.late = 0;
   }
   __syncthreads();
-  const long long tile = S.tile, base = tile * RS_TILE;
+  const long long tile = S.tile, base = tile * TILE;
   if (base >= n) return;  // (block-uniform)
-  const uint32_t mine = group_tile<ARRAY>(S, P, base, n, false);
+  const uint32_t mine = group_tile<ARRAY, ITEMS>(S, P, base, n, false);
   const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
   uint32_t excl = 0;
   if (d < 256) {
@@ -239,7 +252,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_pass(RadixPass P, long 
     S.to[d] = b + excl - S.first[d];
   }
   __syncthreads();
-  const int m = (int)(n - base < RS_TILE ? n - base : RS_TILE);
+  const int m = (int)(n - base < TILE ? n - base : TILE);
 #pragma unroll 4
   for (int i = threadIdx.x; i < m; i += RS_THREADS) {
     const uint32_t key = S.key[i], val = S.val[i], p = S.to[digit_of<ARRAY>(key, val, P.shift, P.len)] + i;
@@ -249,14 +262,15 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_pass(RadixPass P, long 
 }
 
 // up to one tile: all passes in one block
+template <int ITEMS>
 __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_small(RadixPass P, int n, RadixShifts sh) {
   extern __shared__ __align__(16) unsigned char radix_smem[];
-  RadixSmem &S = *reinterpret_cast<RadixSmem *>(radix_smem);
+  RadixSmem<ITEMS> &S = *reinterpret_cast<RadixSmem<ITEMS> *>(radix_smem);
   for (int p = 0; p < sh.n; ++p) {
     P.shift = sh.shift[p];
     P.len = sh.len[p];
-    if (P.len) group_tile<true>(S, P, 0, n, p > 0);
-    else group_tile<false>(S, P, 0, n, p > 0);
+    if (P.len) group_tile<true, ITEMS>(S, P, 0, n, p > 0);
+    else group_tile<false, ITEMS>(S, P, 0, n, p > 0);
     __syncthreads();
   }
   for (int i = threadIdx.x; i < n; i += RS_THREADS) {
@@ -265,34 +279,41 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_small(RadixPass P, int 
   }
 }
 
-template <typename K>
-cudaError_t smem_attr(K k) {
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixSmem));
+template <int ITEMS, typename K>
+cudaError_t radix_smem(K k) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixSmem<ITEMS>));
 }
+template <int ITEMS>
 cudaError_t radix_attr() {
   static const cudaError_t attr = [] {
-    const cudaError_t all[] = {smem_attr(k_radix_small), smem_attr(k_radix_pass<false, uint32_t>), smem_attr(k_radix_pass<true, uint32_t>),
-                               smem_attr(k_radix_pass<false, unsigned long long>), smem_attr(k_radix_pass<true, unsigned long long>)};
+    const cudaError_t all[] = {radix_smem<ITEMS>(k_radix_pass<false, uint32_t, ITEMS>), radix_smem<ITEMS>(k_radix_pass<true, uint32_t, ITEMS>),
+                               radix_smem<ITEMS>(k_radix_pass<false, unsigned long long, ITEMS>),
+                               radix_smem<ITEMS>(k_radix_pass<true, unsigned long long, ITEMS>)};
     for (cudaError_t e : all)
       if (e != cudaSuccess) return e;
     return cudaSuccess;
   }();
   return attr;
 }
+template <int ITEMS>
+cudaError_t radix_run_small(const RadixPass &io, long long n, const RadixShifts &sh, cudaStream_t st) {
+  static const cudaError_t attr = radix_smem<ITEMS>(k_radix_small<ITEMS>);
+  if (attr != cudaSuccess) return attr;
+  k_radix_small<ITEMS><<<1, RS_THREADS, sizeof(RadixSmem<ITEMS>), st>>>(io, (int)n, sh);
+  DMSC_LAUNCHED(1);
+  return cudaGetLastError();
+}
 
 // The passes `sh` from (kin, vin) to (kout, vout); the pairs in between go
 // through t0 and t1 (keys, then values, n words each; t1 only with more than
 // two passes).  The output may be the input.
-cudaError_t radix_run(const RadixPass &io, long long n, const RadixShifts &sh, uint32_t *const t0[2], uint32_t *const t1[2],
+template <int ITEMS>
+cudaError_t radix_run_tiles(const RadixPass &io, long long n, const RadixShifts &sh, uint32_t *const t0[2], uint32_t *const t1[2],
                       cudaStream_t st) {
-  cudaError_t e = radix_attr();
+  constexpr int TILE = RS_THREADS * ITEMS;
+  cudaError_t e = radix_attr<ITEMS>();
   if (e != cudaSuccess) return e;
-  if (n <= RS_TILE) {
-    k_radix_small<<<1, RS_THREADS, sizeof(RadixSmem), st>>>(io, (int)n, sh);
-    DMSC_LAUNCHED(1);
-    return cudaGetLastError();
-  }
-  const long long nt = (n + RS_TILE - 1) / RS_TILE;
+  const long long nt = (n + TILE - 1) / TILE;
   const bool wide = n >= (1ll << 30);
   const size_t words = 256 * (size_t)nt, head = sizeof(uint32_t) * (256 * RS_MAX_PASSES + 2 * RS_MAX_PASSES);
   const size_t wbytes = (wide ? 8 : 4) * words;
@@ -327,12 +348,12 @@ cudaError_t radix_run(const RadixPass &io, long long n, const RadixShifts &sh, u
       q.gather = nullptr;
     }
     auto go = [&](auto kernel, auto *w) {
-      kernel<<<(unsigned)nt, RS_THREADS, sizeof(RadixSmem), st>>>(q, n, hist + 256 * p, w + words * p, counter + p);
+      kernel<<<(unsigned)nt, RS_THREADS, sizeof(RadixSmem<ITEMS>), st>>>(q, n, hist + 256 * p, w + words * p, counter + p);
     };
     uint32_t *w4 = (uint32_t *)(buf + head);
     unsigned long long *w8 = (unsigned long long *)(buf + head);
-    if (wide) q.len ? go(k_radix_pass<true, unsigned long long>, w8) : go(k_radix_pass<false, unsigned long long>, w8);
-    else q.len ? go(k_radix_pass<true, uint32_t>, w4) : go(k_radix_pass<false, uint32_t>, w4);
+    if (wide) q.len ? go(k_radix_pass<true, unsigned long long, ITEMS>, w8) : go(k_radix_pass<false, unsigned long long, ITEMS>, w8);
+    else q.len ? go(k_radix_pass<true, uint32_t, ITEMS>, w4) : go(k_radix_pass<false, uint32_t, ITEMS>, w4);
     DMSC_LAUNCHED(1);
     e = cudaGetLastError();
     k = q.kout;
@@ -340,6 +361,13 @@ cudaError_t radix_run(const RadixPass &io, long long n, const RadixShifts &sh, u
   }
   cudaFreeAsync(buf, st);
   return e;
+}
+
+cudaError_t radix_run(const RadixPass &io, long long n, const RadixShifts &sh, uint32_t *const t0[2], uint32_t *const t1[2],
+                      cudaStream_t st) {
+  if (n <= RS_THREADS * RS_FEW) return radix_run_small<RS_FEW>(io, n, sh, st);
+  if (n <= RS_THREADS * RS_SMALL) return radix_run_small<RS_SMALL>(io, n, sh, st);
+  return n <= RS_FEW_MAX ? radix_run_tiles<RS_FEW>(io, n, sh, t0, t1, st) : radix_run_tiles<RS_ITEMS>(io, n, sh, t0, t1, st);
 }
 
 }  // namespace
@@ -352,7 +380,7 @@ cudaError_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *ktmp, uin
   for (int s = 0; s < nbits && s < 32; s += 8) sh.shift[sh.n++] = s;
   uint32_t *const t[2] = {ktmp, vtmp}, *const o[2] = {keys, vals};
   // through ktmp / vtmp and back; an odd last pass ends there and is copied
-  const bool odd = (sh.n & 1) && n > RS_TILE;
+  const bool odd = (sh.n & 1) && n > radix_tile(n);
   const RadixPass io{keys, vals, odd ? ktmp : keys, odd ? vtmp : vals, nullptr, 0, 0, 0, 0};
   cudaError_t e = radix_run(io, n, sh, t, o, st);
   if (e == cudaSuccess && odd) e = copy_u32(keys, ktmp, n, st);
@@ -379,7 +407,7 @@ cudaError_t sort_pairs_batched(uint32_t *dk, uint32_t *dv, const uint32_t *sk, c
   cudaError_t e = cudaSuccess;
   auto meet = [&](const uint32_t *a, const uint32_t *b) { return a < b + n && b < a + n; };
   const bool inplace_values = batch > 1 && (meet(sv, dk) || meet(sv, dv));  // the last pass gathers from sv while it writes
-  const size_t words = n > RS_TILE ? 4 * (size_t)n : 0, extra = inplace_values ? (size_t)n : 0;
+  const size_t words = n > radix_tile(n) ? 4 * (size_t)n : 0, extra = inplace_values ? (size_t)n : 0;
   if (words + extra) e = cudaMallocAsync((void **)&buf, sizeof(uint32_t) * (words + extra), st);
   if (e != cudaSuccess) return e;
   uint32_t *const t0[2] = {buf, buf + n}, *const t1[2] = {buf + 2 * n, buf + 3 * n};
