@@ -205,7 +205,7 @@ struct MergeJob {
   dmsc_msc *a, *b, *parent;
   int ixn[4];
 };
-// seq_ms accumulates the host wall time of the one-thread steps.
+// seq_ms accumulates the host wall time of the boundary steps.
 cudaError_t merge_up_level_par(const std::vector<MergeJob> &jobs, unsigned long long grow, uint32_t *status,
                                uint32_t *stw, cudaStream_t st, double *seq_ms, long long round_window,
                                long long round_min_commits);

@@ -575,7 +575,7 @@ struct SeqJob {
   int win = 0, min_commits = 0;  // SEQ_UP_CANCEL: rounds window (0: groups of cells) and hand-off rate
 };
 
-// Loads, across the GPU, what the one-thread step of a job will read -- the
+// Loads, across the GPU, what the boundary step of a job will read -- the
 // boundary points, their partners, their lists and their neighbours' list
 // descriptors -- so that the step finds it in L2 instead of DRAM.  Reads
 // only; the sum is stored only under a condition that never holds, so the
