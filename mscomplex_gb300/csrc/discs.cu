@@ -18,6 +18,7 @@
 // chains (section 4b below) placed window by window, with one block per saddle
 // that grows its disc level by level (the output array as the queue) for the
 // few saddles with more than KMAX chains.
+#include "chain_walk.h"
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 #include "grid_types.h"
@@ -258,7 +259,6 @@ __device__ __forceinline__ uint32_t seed_cell(const DiscArgs &a, const SeedRuns 
 // that reach it one lane each, and stores the window out (k_win_place).
 // ---------------------------------------------------------------------------
 constexpr int KMAX = 32;                 // saddles with more chains grow level by level (k_big_discs)
-constexpr uint32_t HOP_END = 0xFFFFFFFFu;
 constexpr int HOP_SLOTS = 2 * TX * TY;   // H and Vt edge of every vertex of a tile
 constexpr uint16_t SLOT_NIL = 0xFFFF;
 
@@ -363,7 +363,6 @@ __device__ __forceinline__ int chain_kind(uint32_t code, int rx, int ry) {
 constexpr int HOP_THREADS = 512;
 // successor of an edge along its chain as a step code (0-5, as in the successor words)
 constexpr uint8_t SUCC_NONE = 0xFF;
-constexpr int SEG_LOG = 5, SEG_MAX = 1 << SEG_LOG;  // cells of a write piece: the jump pointer distance
 
 constexpr uint8_t SUCC_TWO = 0xFE;  // a cell with two successors (it ends no chain)
 struct HopSmem {
@@ -596,25 +595,10 @@ __global__ void k_chain_count(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
   }
 }
 
-// The chain from ext-local edge e: its length, stored with its piece count as
-// chain j of saddle s where that saddle's chains are kept.
-__device__ __forceinline__ unsigned long long chain_walk(const DiscArgs &a, const ChainArgs &c, uint32_t s, uint32_t j, uint32_t e) {
-  unsigned long long L = 0;
-  uint32_t nseg = 0;
-  for (uint32_t x = e; x != HOP_END; x = c.hop_to[x]) {
-    const uint32_t l = c.hop_len[x];
-    if (l == 0) { atomicOr(a.status, ST_INVARIANT); break; }  // a chain cell never branches
-    L += l;
-    nseg += (l + SEG_MAX - 1) / SEG_MAX;
-    if (L > c.limit) { atomicOr(a.status, ST_CYCLE); return 0; }
-  }
-  if (!(c.big[s] & 1u)) {
-    // piece slots: one per SEG_MAX cells of each hop, and one more for each level
-    // where another of the saddle's chains ends inside this one (at most K - 1)
-    if (j < c.cap) { c.cstart[j] = e; c.csaddle[j] = s; c.clen[j] = (uint32_t)L; c.cnseg[j] = nseg + c.kc[s] - 1; }
-    else atomicOr(a.status, ST_CAPACITY);
-  }
-  return L;
+__device__ __forceinline__ void chain_fault(const DiscArgs &a, uint32_t fault) {
+  if (fault)
+    atomicOr(a.status, (fault & CHAIN_BRANCHES ? ST_INVARIANT : 0u) | (fault & CHAIN_CYCLE ? ST_CYCLE : 0u) |
+                           (fault & CHAIN_NO_SLOT ? ST_CAPACITY : 0u));
 }
 // the chains of every saddle's own seeds
 __global__ void k_chain_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
@@ -625,10 +609,12 @@ __global__ void k_chain_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
     uint32_t seed[4], ch[2];
     const int own = own_seeds(a, kind, a.cellid[s], seed);
     unsigned long long total = 0;
+    uint32_t fault = 0;
     for (int q = 0; q < own; ++q) {
       const int n = item_children(a, kind, seed[q], ch);
-      for (int b = 0; b < n; ++b) total += chain_walk(a, c, s, j++, ch[b]);
+      for (int b = 0; b < n; ++b) total += chain_walk(c, s, j++, ch[b], fault);
     }
+    chain_fault(a, fault);
     c.dlen[s] += total;
   }
 }
@@ -641,7 +627,9 @@ __global__ void k_seed_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
       uint32_t j = c.cbase[s] + sr.chains[p] - sr.chains[sr.start[s]] + (sr.val[p] < s ? 0u : (c.big[s] >> 1) & 15u);
       uint32_t ch[2];
       const int n = item_children(a, kind, seed_cell(a, sr, p), ch);
-      for (int b = 0; b < n; ++b) total += chain_walk(a, c, s, j++, ch[b]);
+      uint32_t fault = 0;
+      for (int b = 0; b < n; ++b) total += chain_walk(c, s, j++, ch[b], fault);
+      chain_fault(a, fault);
     }
     // items are sorted by saddle: one addition for a warp's items of one saddle
     const unsigned m = __activemask(), same = __match_any_sync(m, s);
