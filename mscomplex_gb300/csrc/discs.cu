@@ -157,9 +157,10 @@ __global__ void k_seed_count(DiscArgs a, int kind, uint32_t *cnt) {
     cnt[i] = c;
   }
 }
-// (one thread per item: a cancelled extremum's list may hold most of them)
+// (one thread per item: a cancelled extremum's list may hold most of them; the
+// loops over the items have 64-bit indices, as there may be nearly 2^32)
 __global__ void k_seed_write(DiscArgs a, int kind, const uint32_t *off, uint32_t n, uint32_t *key, uint32_t *val) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+  for (unsigned long long p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = a.ncp;  // the last point whose items start at or before p
     while (hi - lo > 1) {
       const uint32_t m = lo + (hi - lo) / 2;
@@ -228,7 +229,7 @@ __device__ __forceinline__ uint32_t pushes_before(const SeedRuns &sr, uint32_t s
   uint32_t lo = 0, hi = sr.count[s];
   const uint32_t *v = sr.val + (hi ? sr.start[s] : 0);
   while (lo < hi) {
-    const uint32_t m = (lo + hi) >> 1;
+    const uint32_t m = lo + (hi - lo) / 2;
     if (v[m] < s) lo = m + 1; else hi = m;
   }
   return lo;
@@ -568,7 +569,7 @@ __device__ __forceinline__ int item_children(const DiscArgs &a, int kind, uint32
 
 // chains that each item starts
 __global__ void k_seed_chains(DiscArgs a, int kind, SeedRuns sr, uint32_t *cnt) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+  for (unsigned long long p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
     const uint32_t s = sr.key[p];
     uint32_t ch[2];
     cnt[p] = s < a.ncp && surviving_saddle(a, s) ? (uint32_t)item_children(a, kind, seed_cell(a, sr, p), ch) : 0u;
@@ -620,7 +621,7 @@ __global__ void k_chain_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
 }
 // the chains of the items from cancelled extrema
 __global__ void k_seed_len(DiscArgs a, int kind, SeedRuns sr, ChainArgs c) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+  for (unsigned long long p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
     const uint32_t s = sr.key[p];
     unsigned long long total = 0;
     if (s < a.ncp && surviving_saddle(a, s)) {
@@ -732,7 +733,7 @@ __global__ void k_level0(DiscArgs a, int kind, SeedRuns sr, const uint32_t *off,
   }
 }
 __global__ void k_seed_level0(DiscArgs a, SeedRuns sr, ChainArgs c, const uint32_t *off, uint32_t *out) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
+  for (unsigned long long p = blockIdx.x * blockDim.x + threadIdx.x; p < sr.n; p += gridDim.x * blockDim.x) {
     const uint32_t s = sr.key[p];
     if (s >= a.ncp || !surviving_saddle(a, s)) continue;
     const uint32_t o = off[s] + (p - sr.start[s]) + (sr.val[p] < s ? 0u : c.big[s] >> 5);
