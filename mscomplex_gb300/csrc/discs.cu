@@ -22,6 +22,7 @@
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 #include "grid_types.h"
+#include "smem_limit.h"
 #include <algorithm>
 
 namespace dmsc {
@@ -1107,9 +1108,8 @@ static int nbits_for(long long n) {
 }
 
 static cudaError_t hops_attr() {
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_disc_hops, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HopSmem));
-  return attr;
+  static SmemLimit limit;
+  return limit.raise(sizeof(HopSmem), k_disc_hops);
 }
 
 // Everything both disc kinds share: the hop structure, the redirections, the

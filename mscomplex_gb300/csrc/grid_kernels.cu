@@ -53,6 +53,7 @@
 
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
+#include "smem_limit.h"
 
 namespace dmsc {
 
@@ -781,9 +782,9 @@ size_t label_smem_bytes() { return sizeof(LabelSmem); }
 
 cudaError_t launch_gradient(const float *hgt, const GridGeom &g, uint32_t *codes, uint32_t *terms, uint8_t *rowcnt,
                             uint64_t *table, uint32_t *status, cudaStream_t st) {
-  // once per process (thread-safe static initialisation)
-  static const cudaError_t attr = cudaFuncSetAttribute(k_gradient, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(sizeof(GradSmem), k_gradient);
+  if (e != cudaSuccess) return e;
   dim3 grid(g.ntx, g.nty);
   k_gradient<<<grid, GRAD_THREADS, sizeof(GradSmem), st>>>(hgt, g, codes, terms, rowcnt, table, status);
   DMSC_LAUNCHED(1);
@@ -804,9 +805,9 @@ cudaError_t launch_resolve(uint64_t *table, long long nslots, const uint32_t *of
 cudaError_t launch_labels(const uint32_t *codes, const uint32_t *terms, const float *hgt, const GridGeom &g,
                           const uint32_t *offsets, const uint64_t *table, uint4 *labels, const CpOut &cp,
                           uint32_t *status, cudaStream_t st) {
-  // once per process (thread-safe static initialisation)
-  static const cudaError_t attr = cudaFuncSetAttribute(k_labels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LabelSmem));
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(sizeof(LabelSmem), k_labels);
+  if (e != cudaSuccess) return e;
   dim3 grid(g.ntx, g.nty);
   k_labels<<<grid, GRAD_THREADS, sizeof(LabelSmem), st>>>(codes, terms, hgt, g, offsets, table, labels, cp, status);
   DMSC_LAUNCHED(1);
@@ -830,9 +831,9 @@ static long long persistent_blocks(long long ntiles, int blocks_per_sm) {
 template <int THREADS>
 static cudaError_t gradient_batch_t(const BatchGrid *grids, int ngrids, long long ntiles, int bps, uint32_t *status,
                                     cudaStream_t st) {
-  static const cudaError_t attr =  // once per instantiation (thread-safe static initialisation)
-      cudaFuncSetAttribute(k_gradient_batch<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(sizeof(GradSmem), k_gradient_batch<THREADS>);
+  if (e != cudaSuccess) return e;
   k_gradient_batch<THREADS><<<(unsigned)persistent_blocks(ntiles, bps), THREADS, sizeof(GradSmem), st>>>(grids, ngrids,
                                                                                                       ntiles, status);
   DMSC_LAUNCHED(1);
@@ -842,9 +843,9 @@ static cudaError_t gradient_batch_t(const BatchGrid *grids, int ngrids, long lon
 template <int THREADS>
 static cudaError_t labels_batch_t(const BatchGrid *grids, int ngrids, long long ntiles, const CpOut &cp, int bps,
                                   uint32_t *status, cudaStream_t st) {
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_labels_batch<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LabelSmem));
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(sizeof(LabelSmem), k_labels_batch<THREADS>);
+  if (e != cudaSuccess) return e;
   k_labels_batch<THREADS><<<(unsigned)persistent_blocks(ntiles, bps), THREADS, sizeof(LabelSmem), st>>>(grids, ngrids,
                                                                                                      ntiles, cp, status);
   DMSC_LAUNCHED(1);

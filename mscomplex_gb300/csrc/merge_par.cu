@@ -45,6 +45,7 @@
 #include "grid_types.h"
 #include "host_pool.h"
 #include "merge_graph.cuh"
+#include "smem_limit.h"
 #include "warp_graph.cuh"
 
 namespace dmsc {
@@ -1372,15 +1373,13 @@ cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob>
   if (e == cudaSuccess) {
     k_seq_prefetch<<<dim3(64, (unsigned)nj), 256, 0, st>>>(dg, dj, nullptr);
     if (rounds) {
-      static const cudaError_t attr = cudaFuncSetAttribute(k_merge_up_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           (int)sizeof(RoundSmem));
-      e = attr;
+      static SmemLimit limit;
+      e = limit.raise(sizeof(RoundSmem), k_merge_up_rounds);
       if (e == cudaSuccess)
         k_merge_up_rounds<<<(unsigned)nj, ROUND_THREADS, sizeof(RoundSmem), st>>>(dg, dj, (int)nj, dslot, status);
     } else if (down) {
-      static const cudaError_t attr =
-          cudaFuncSetAttribute(k_merge_down_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DOWN_SMEM);
-      e = attr;
+      static SmemLimit limit;
+      e = limit.raise(DOWN_SMEM, k_merge_down_seq);
       if (e == cudaSuccess)
         k_merge_down_seq<<<(unsigned)nj, 32 * DOWN_WARPS, DOWN_SMEM, st>>>(dg, dj, (int)nj, (const DownWork *)(buf + head), status);
     } else {

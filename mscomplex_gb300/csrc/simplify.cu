@@ -24,6 +24,7 @@
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
 #include "msc_graph.cuh"
+#include "smem_limit.h"
 #include "warp_graph.cuh"
 
 #include <algorithm>
@@ -777,12 +778,10 @@ static cudaError_t launch_simplify(SimpArgs *args, int n, int levels, cudaStream
   const int warps = n <= 152 ? 16 : 8;
   const uint32_t own = n <= 152 ? 1024 : 512, shared = n <= 152 ? 8192 : 4096;
   constexpr size_t un_max = sizeof(uint2) * (16 * 1024 + 8192) + sizeof(uint32_t) * DONE_WORDS;
-  static const cudaError_t attr = [] {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_simplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)top_bytes(TOP_LEVELS));
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_unsimplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)un_max);
-  }();
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit, un_limit;
+  cudaError_t e = limit.raise(top_bytes(TOP_LEVELS), k_simplify);
+  if (e == cudaSuccess) e = un_limit.raise(un_max, k_unsimplify);
+  if (e != cudaSuccess) return e;
   k_simplify<<<n, 32 * SIMP_WARPS, top_bytes(levels), st>>>(args, n, levels);
   k_unsimplify<<<n, 32 * warps, sizeof(uint2) * (warps * own + shared) + sizeof(uint32_t) * DONE_WORDS, st>>>(args, n, own, shared);
   k_entry_sums<<<dim3(n == 1 ? 64 : 4, n), 256, 0, st>>>(args);

@@ -19,6 +19,7 @@
 // us with 20 a thread, 51 so; 6,000: 104, 61).
 #include "dmsc_common.cuh"
 #include "dmsc_internal.h"
+#include "smem_limit.h"
 
 #include <algorithm>
 
@@ -279,26 +280,11 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_radix_small(RadixPass P, int 
   }
 }
 
-template <int ITEMS, typename K>
-cudaError_t radix_smem(K k) {
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixSmem<ITEMS>));
-}
-template <int ITEMS>
-cudaError_t radix_attr() {
-  static const cudaError_t attr = [] {
-    const cudaError_t all[] = {radix_smem<ITEMS>(k_radix_pass<false, uint32_t, ITEMS>), radix_smem<ITEMS>(k_radix_pass<true, uint32_t, ITEMS>),
-                               radix_smem<ITEMS>(k_radix_pass<false, unsigned long long, ITEMS>),
-                               radix_smem<ITEMS>(k_radix_pass<true, unsigned long long, ITEMS>)};
-    for (cudaError_t e : all)
-      if (e != cudaSuccess) return e;
-    return cudaSuccess;
-  }();
-  return attr;
-}
 template <int ITEMS>
 cudaError_t radix_run_small(const RadixPass &io, long long n, const RadixShifts &sh, cudaStream_t st) {
-  static const cudaError_t attr = radix_smem<ITEMS>(k_radix_small<ITEMS>);
-  if (attr != cudaSuccess) return attr;
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(sizeof(RadixSmem<ITEMS>), k_radix_small<ITEMS>);
+  if (e != cudaSuccess) return e;
   k_radix_small<ITEMS><<<1, RS_THREADS, sizeof(RadixSmem<ITEMS>), st>>>(io, (int)n, sh);
   DMSC_LAUNCHED(1);
   return cudaGetLastError();
@@ -311,7 +297,9 @@ template <int ITEMS>
 cudaError_t radix_run_tiles(const RadixPass &io, long long n, const RadixShifts &sh, uint32_t *const t0[2], uint32_t *const t1[2],
                       cudaStream_t st) {
   constexpr int TILE = RS_THREADS * ITEMS;
-  cudaError_t e = radix_attr<ITEMS>();
+  static SmemLimit limit;
+  cudaError_t e = limit.raise(sizeof(RadixSmem<ITEMS>), k_radix_pass<false, uint32_t, ITEMS>, k_radix_pass<true, uint32_t, ITEMS>,
+                              k_radix_pass<false, unsigned long long, ITEMS>, k_radix_pass<true, unsigned long long, ITEMS>);
   if (e != cudaSuccess) return e;
   const long long nt = (n + TILE - 1) / TILE;
   const bool wide = n >= (1ll << 30);
