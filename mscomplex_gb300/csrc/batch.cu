@@ -336,6 +336,9 @@ int dmsc_batch_run(dmsc_ctx *ctx, int ngrids, const int32_t *sizes, const float 
         if (s == ST_SIMPLIFY_LIMIT && B->stats[5 * g + 3] <= io.max_ops) {
           B->gstat[g] = DMSC_ERR_DEVICE_TIMEOUT;
           B->gerr[g] = "grid " + std::to_string(g) + ": simplification ran out of list pool after retries";
+        } else if (s & ST_WAIT_LIMIT) {
+          B->gstat[g] = DMSC_ERR_DEVICE_TIMEOUT;
+          B->gerr[g] = "grid " + std::to_string(g) + ": simplification waited for a list that nobody was working on";
         } else if (s & ST_TOO_LONG) {
           B->gstat[g] = DMSC_ERR_OOM;
           B->gerr[g] = "grid " + std::to_string(g) + ": lists of more than 2^32 - 1 entries";

@@ -47,6 +47,7 @@ static int status_to_error(uint32_t st) {
   if (!st) return DMSC_OK;
   if (st & ST_NAN_INPUT) return fail(DMSC_ERR_INPUT, "NaN height in input (outside the supported domain)");
   if (st & ST_TOO_LONG) return fail(DMSC_ERR_OOM, "lists or discs of more than 2^32 - 1 entries");
+  if (st & ST_WAIT_LIMIT) return fail(DMSC_ERR_DEVICE_TIMEOUT, "a warp waited for a list that nobody was working on");
   if (st & (ST_RESOLVE_LIMIT | ST_SIMPLIFY_LIMIT))
     return fail(DMSC_ERR_DEVICE_TIMEOUT, "a bounded device loop ran out of iterations (status " + std::to_string(st) + ")");
   return fail(DMSC_ERR_INVARIANT, "device invariant violated (status " + std::to_string(st) + ")");

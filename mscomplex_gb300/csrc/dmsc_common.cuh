@@ -36,8 +36,9 @@ enum : uint32_t {
   ST_SIMPLIFY_LIMIT = 1u << 5, // simplification pool / iteration bound exceeded
   ST_INVARIANT = 1u << 6,      // a reference logic_error condition (merge / disc invariants)
   ST_CAPACITY = 1u << 7,       // critical-point arrays too small (host grows them and reruns)
-  ST_TOO_LONG = 1u << 9,       // lists or discs hold more entries than their 32-bit offsets count
   ST_FALLBACK = 1u << 8,       // a parallel merge met a case only the one-thread restatement reproduces
+  ST_TOO_LONG = 1u << 9,       // lists or discs hold more entries than their 32-bit offsets count
+  ST_WAIT_LIMIT = 1u << 10,    // a warp waited for another one's list while no warp got on (never expected)
 };
 
 constexpr uint32_t LABEL_NONE = 0xFFFFFFFFu;

@@ -960,7 +960,7 @@ __global__ void __launch_bounds__(32 * DOWN_WARPS, 1) k_merge_down_seq(MGraph *g
   if (threadIdx.x == 0) {
     team.top = M.G.L.top;
     team.shared_top = nullptr;
-    team.fail = team.wrong = 0;
+    team.fail = team.wrong = team.late = team.beat = 0;
     team.lock = 0;
     odd = n > DOWN_CELLS;
   }
@@ -1047,7 +1047,8 @@ __global__ void __launch_bounds__(32 * DOWN_WARPS, 1) k_merge_down_seq(MGraph *g
     MGraph g = M;
     g.G.fail = team.fail != 0 && !team.wrong;
     g.G.L.top = team.top;
-    if (team.wrong) set_status(status, ST_INVARIANT);  // (the other warps stopped for it)
+    if (team.late) set_status(status, ST_WAIT_LIMIT);
+    else if (team.wrong) set_status(status, ST_INVARIANT);  // (the other warps stopped for it)
     else if (team.fail) set_status(status, ST_SIMPLIFY_LIMIT);
     graphs[jb.g0] = g;
   }

@@ -178,6 +178,7 @@ static int run_level_par(dmsc_pipeline *P, bool up, const std::vector<int> &node
         for (auto &J : jobs) J.parent->ncp = J.parent->nasc = J.parent->ndes = 0;
       return LEVEL_FALLBACK;
     }
+    if (stw & ST_WAIT_LIMIT) return perr(DMSC_ERR_DEVICE_TIMEOUT, "a merge waited for a list that nobody was working on");
     if (stw == ST_SIMPLIFY_LIMIT && attempt + 1 < 4) continue;
     if (stw & ST_SIMPLIFY_LIMIT) return perr(DMSC_ERR_DEVICE_TIMEOUT, "a merge ran out of list pool or table room");
     if (stw) return perr(DMSC_ERR_INVARIANT, "merge invariant violated (status " + std::to_string(stw) + ")");

@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(32 * SIMP_WARPS, 2) k_simplify(SimpArgs *args,
     sh.team.top = a.G.L.top;
     sh.team.shared_top = nullptr;
     sh.team.ops = 0;
-    sh.team.fail = sh.team.wrong = 0;
+    sh.team.fail = sh.team.wrong = sh.team.late = sh.team.beat = 0;
     sh.stop = 0;
   }
   __syncthreads();
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, ui
     team.shared_top = nullptr;
     team.ops = a.G.ops;
     team.ticket = 2ull * a.ncanc;
-    team.fail = team.wrong = 0;
+    team.fail = team.wrong = team.late = team.beat = 0;
     team.lock = 0;
   }
   for (uint32_t i = threadIdx.x; i < a.G.ncp; i += blockDim.x) a.meta[i] = 0;
@@ -749,7 +749,8 @@ __global__ void __launch_bounds__(512, 1) k_unsimplify(SimpArgs *args, int n, ui
   __syncthreads();
   if (threadIdx.x == 0) {
     a.stats[3] = team.ops;
-    if (team.wrong) a.stats[4] |= ST_INVARIANT;  // (the other warps stopped for it)
+    if (team.late) a.stats[4] |= ST_WAIT_LIMIT;
+    else if (team.wrong) a.stats[4] |= ST_INVARIANT;  // (the other warps stopped for it)
     else if (team.fail || team.ops > a.G.max_ops) a.stats[4] |= ST_SIMPLIFY_LIMIT;
   }
 }

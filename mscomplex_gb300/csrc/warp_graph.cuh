@@ -46,9 +46,19 @@ struct TeamState {
   unsigned long long ticket; // pairs not yet taken
   uint32_t fail, wrong;      // a pool, budget or wait ran out; a reference logic_error condition
   int lock;                  // 1: a warp uses the scratch all warps share
+  uint32_t late;             // a wait on another warp ran out (fail is set too)
+  uint32_t beat;             // changes while any warp gets on with its work
   unsigned long long *shared_top;  // the pool's top where several blocks edit the graph (then top is unused)
 };
-constexpr unsigned long long WAIT_LIMIT = 1ull << 26;  // polls of a wait on another warp
+// A wait on another warp ends after so many polls during which no warp of the
+// team got on.  (A list may take longer than that to rewrite: millions of
+// values are sorted by one warp in global memory, at worst by one lane.  Its
+// loops move the team's beat on at least every few ms.)
+#ifndef DMSC_WAIT_POLLS
+#define DMSC_WAIT_POLLS (1ull << 26)
+#endif
+constexpr unsigned long long WAIT_LIMIT = DMSC_WAIT_POLLS;
+constexpr uint32_t BEAT_STEPS = 4096;  // steps of a loop over a list between two beats (a power of two)
 constexpr int BAR_EDIT = 3;
 
 struct WarpGraph {
@@ -66,6 +76,27 @@ struct WarpGraph {
   uint32_t nshared_stage = 0;
 
   __device__ __forceinline__ unsigned lt() const { return (1u << lane) - 1u; }
+  // the calling lane's warp has got on with its work
+  __device__ __forceinline__ void moved_on() const {
+    if (team) atomicAdd(&team->beat, 1u);
+  }
+  // One more poll of a wait on another warp: whether to give up.  polls is 0
+  // before the first one; beat is the wait's own.
+  __device__ __forceinline__ bool give_up(unsigned long long &polls, uint32_t &beat) const {
+    if (*(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong) return true;
+    if (polls != 0 && polls < WAIT_LIMIT) {
+      ++polls;
+      return false;
+    }
+    const uint32_t now = *(volatile uint32_t *)&team->beat;
+    if (polls != 0 && now == beat) {
+      *(volatile uint32_t *)&team->late = 1;
+      return true;
+    }
+    beat = now;
+    polls = 1;
+    return false;
+  }
 
   // first run of p[0..n) (ascending values) with value >= x
   __device__ __forceinline__ uint32_t lower(const uint2 *p, uint32_t n, uint32_t x) const {
@@ -647,6 +678,7 @@ struct WarpGraph {
         for (unsigned long long j = k >> 1; j > 0; j >>= 1) {
 #pragma unroll 4
           for (unsigned long long t = lane; t < N / 2; t += 32) {
+            if ((t & (BEAT_STEPS * 32 - 1)) == 0) moved_on();  // (lane 0)
             const unsigned long long i = 2 * t - (t & (j - 1)), o = i + j;  // the t-th pair at distance j
             const uint2 x = b[i], y = b[o];
             if ((x.x > y.x) == ((i & k) == 0)) { b[i] = y; b[o] = x; }
@@ -654,13 +686,28 @@ struct WarpGraph {
           __syncwarp();
         }
     } else {
-      if (lane == 0) G.sort_tmp(n);
+      if (lane == 0) {  // heap sort, as Graph::sort_tmp
+        for (unsigned long long s = n / 2; s-- > 0;) {
+          if ((s & 1023) == 0) moved_on();
+          G.sift(s, n);
+        }
+        for (unsigned long long e = n; e-- > 1;) {
+          if ((e & 1023) == 0) moved_on();
+          const uint2 q = b[0];
+          b[0] = b[e];
+          b[e] = q;
+          G.sift(0, e);
+        }
+      }
       __syncwarp();
     }
     // equal neighbours become one run
     auto is_head = [&](unsigned long long u) { return u < n && (u == 0 || b[u - 1].x != b[u].x); };
     uint32_t m = 0;
-    for (unsigned long long u0 = 0; u0 < n; u0 += 32) m += __popc(__ballot_sync(FULL_WARP, is_head(u0 + lane)));
+    for (unsigned long long u0 = 0; u0 < n; u0 += 32) {
+      if (lane == 0 && (u0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
+      m += __popc(__ballot_sync(FULL_WARP, is_head(u0 + lane)));
+    }
     uint32_t off = G.L.off[l];
     if (m > cap && !grow(l, cap, m, off)) return false;
     uint2 *p = G.L.pool + off;
@@ -668,13 +715,17 @@ struct WarpGraph {
     bool bad = false;
     uint32_t w = 0;
     for (unsigned long long u0 = 0; u0 < n; u0 += 32) {
+      if (lane == 0 && (u0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
       const unsigned long long u = u0 + lane;
       const bool head = is_head(u);
       const unsigned hb = __ballot_sync(FULL_WARP, head);
       if (head) {
         const uint32_t x = b[u].x;
         unsigned long long s = 0;
-        for (unsigned long long q = u; q < n && b[q].x == x; ++q) s += b[q].y;
+        for (unsigned long long q = u; q < n && b[q].x == x; ++q) {
+          if ((q - u) % BEAT_STEPS == BEAT_STEPS - 1) moved_on();
+          s += b[q].y;
+        }
         if (s > 0xffffffffull) bad = true;
         tot += s;
         p[w + __popc(hb & lt())] = make_uint2(x, (uint32_t)s);
@@ -734,8 +785,10 @@ struct WarpGraph {
             cancelled = o <= turn;
             const uint32_t bit = 2 * (o - 1) + i;
             volatile const uint32_t *w = done + (bit >> 5);
-            for (unsigned long long polls = 0; !cancelled && !((*w >> (bit & 31)) & 1u);)
-              if (++polls > WAIT_LIMIT || *(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong) {
+            unsigned long long polls = 0;
+            uint32_t beat = 0;
+            while (!cancelled && !((*w >> (bit & 31)) & 1u))
+              if (give_up(polls, beat)) {
                 t.stopped = true;  // the wait ran out, or another warp's pair failed
                 break;
               }
@@ -773,7 +826,10 @@ struct WarpGraph {
       const int s = __ffs(lg) - 1;
       const uint32_t sc = __shfl_sync(FULL_WARP, t.cnt, s), ss = __shfl_sync(FULL_WARP, t.src, s);
       const uint32_t so = __shfl_sync(FULL_WARP, o, s), sy = __shfl_sync(FULL_WARP, t.run.y, s);
-      for (uint32_t q = lane; q < sc; q += 32) one(G.L.pool[ss + q], sy, so + q);
+      for (uint32_t q = lane; q < sc; q += 32) {
+        if ((q & (BEAT_STEPS * 32 - 1)) == 0) moved_on();  // (lane 0)
+        one(G.L.pool[ss + q], sy, so + q);
+      }
     }
     return all;
   }
@@ -786,10 +842,10 @@ struct WarpGraph {
     if (team) {
       bool got = false;
       if (lane == 0) {
-        for (unsigned long long polls = 0; !got && polls <= WAIT_LIMIT; ++polls) {
-          got = atomicCAS(&team->lock, 0, 1) == 0;
-          if (!got && (*(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong)) break;
-        }
+        unsigned long long polls = 0;
+        uint32_t beat = 0;
+        do got = atomicCAS(&team->lock, 0, 1) == 0;
+        while (!got && !give_up(polls, beat));
         __threadfence_block();
       }
       if (!__shfl_sync(FULL_WARP, got, 0)) { G.fail = true; return nullptr; }
@@ -852,6 +908,7 @@ struct WarpGraph {
     } else {
       if (!holds(p, nr, other)) return false;
       for (uint32_t k0 = 0; k0 < nr; k0 += 32) {  // the items' number, and the checks
+        if (lane == 0 && (k0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
         const Item t = item_of(p, nr, k0 + lane, other, i, turn);
         wrong |= t.wrong;
         bad |= t.stopped;
@@ -892,7 +949,10 @@ struct WarpGraph {
       }
       __threadfence_block();
       __syncwarp();
-      if (lane == 0) atomicOr(&done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
+      if (lane == 0) {
+        atomicOr(&done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
+        moved_on();
+      }
     }
   }
 };
