@@ -105,7 +105,6 @@ struct SimplifyIO {
   int rect[4] = {0, 0, 0, 0};
   double tresh = 0;
   unsigned long long max_ops = 0;
-  unsigned long long heap_cap = 0, tmp_cap = 0, pool_extra = 0;  // 0 = defaults
   unsigned long long *host_stats = nullptr;  // pinned, 8 words: [0] pushes [1] pops [2] cancels [3] ops [4] status [5] asc [6] des entries
   long long nasc_out = 0, ndes_out = 0;
   void *work = nullptr;

@@ -46,33 +46,23 @@ __device__ __forceinline__ uint32_t block_exscan(uint32_t v, uint32_t &excl) {
   return total;
 }
 
-// A thread's SCAN_ITEMS consecutive items: one or two vector loads when the
-// array is aligned for them and the items are all in range, else scalars.
-template <typename T>
-__device__ __forceinline__ void load_items(const T *__restrict__ in, long long base, long long n, bool vec,
+// The scan with the caller's scratch (scan_exclusive_u32_scratch): a thread's
+// SCAN_ITEMS consecutive items, by two vector loads when the array is aligned
+// for them and the items are all in range, else scalars.
+__device__ __forceinline__ void load_items(const uint32_t *__restrict__ in, long long base, long long n, bool vec,
                                            uint32_t v[SCAN_ITEMS]) {
-  static_assert(SCAN_ITEMS == 8, "two 16-byte (u32) or one 8-byte (u8) vector per thread");
+  static_assert(SCAN_ITEMS == 8, "two 16-byte vectors per thread");
   if (vec && base + SCAN_ITEMS <= n) {
-    if constexpr (sizeof(T) == 4) {
-      const uint4 a = reinterpret_cast<const uint4 *>(in + base)[0], b = reinterpret_cast<const uint4 *>(in + base)[1];
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
-      const uint2 a = *reinterpret_cast<const uint2 *>(in + base);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { v[k] = (a.x >> (8 * k)) & 0xffu; v[4 + k] = (a.y >> (8 * k)) & 0xffu; }
-    }
+    const uint4 a = reinterpret_cast<const uint4 *>(in + base)[0], b = reinterpret_cast<const uint4 *>(in + base)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     return;
   }
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = (base + k < n) ? (uint32_t)in[base + k] : 0u;
+  for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = base + k < n ? in[base + k] : 0u;
 }
-template <typename T>
-__host__ __forceinline__ bool items_aligned(const T *p) {
-  return ((uintptr_t)p % (sizeof(T) == 4 ? 16 : 8)) == 0;
-}
+__host__ __forceinline__ bool items_aligned(const uint32_t *p) { return (uintptr_t)p % 16 == 0; }
 
-template <typename T>
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const T *__restrict__ in, long long n, bool vec,
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__restrict__ in, long long n, bool vec,
                                                               uint32_t *partial) {
   long long base = (long long)blockIdx.x * SCAN_CHUNK + (long long)threadIdx.x * SCAN_ITEMS;
   uint32_t v[SCAN_ITEMS];
@@ -87,8 +77,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const T *__restric
 
 // (in and out may be the same array: a thread reads its items before it
 // writes them, and no thread reads another's)
-template <typename T>
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const T *in, long long n, bool vec_in,
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t *in, long long n, bool vec_in,
                                                             const uint32_t *__restrict__ block_off, uint32_t *out,
                                                             bool vec_out, uint32_t *total) {
   long long base = (long long)blockIdx.x * SCAN_CHUNK + (long long)threadIdx.x * SCAN_ITEMS;
@@ -341,17 +330,16 @@ cudaError_t scan_exclusive_u32_scratch(const uint32_t *in, long long n, uint32_t
   }
   long long nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
   if (nb == 1) {
-    k_scan_down<uint32_t><<<1, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), nullptr, out, items_aligned(out), total);
+    k_scan_down<<<1, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), nullptr, out, items_aligned(out), total);
     DMSC_LAUNCHED(1);
     return cudaGetLastError();
   }
   uint32_t *part = scratch, *poff = scratch + nb;
-  k_scan_reduce<uint32_t><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), part);
+  k_scan_reduce<<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), part);
   DMSC_LAUNCHED(1);
   cudaError_t e = scan_exclusive_u32_scratch(part, nb, poff, nullptr, scratch + 2 * nb, st);
   if (e != cudaSuccess) return e;
-  k_scan_down<uint32_t><<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), poff, out,
-                                                                items_aligned(out), total);
+  k_scan_down<<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, items_aligned(in), poff, out, items_aligned(out), total);
   DMSC_LAUNCHED(1);
   return cudaGetLastError();
 }

@@ -898,10 +898,10 @@ cudaError_t simplify_run(SimplifyIO &io, cudaStream_t st) {
   const uint32_t ncp = (uint32_t)io.ncp;
   unsigned long long des_base = (unsigned long long)io.nasc + 4ull * ncp;
   unsigned long long base_top = des_base + (unsigned long long)io.ndes + 4ull * ncp;
-  unsigned long long pool_cap = base_top + (io.pool_extra ? io.pool_extra : (2 * base_top + (1ull << 22)));
-  const unsigned long long heap_cap = std::min(io.heap_cap ? io.heap_cap : (4ull * io.ndes + (1ull << 20)), HEAP_MAX);
+  const unsigned long long pool_cap = base_top + 2 * base_top + (1ull << 22);
+  const unsigned long long heap_cap = std::min(4ull * io.ndes + (1ull << 20), HEAP_MAX);
   // scratch runs: two per added value of a merged list (edit_list), per helper warp
-  unsigned long long tmp_cap = io.tmp_cap ? io.tmp_cap : std::max(1ull << 22, 2ull * HELPERS * ncp);
+  const unsigned long long tmp_cap = std::max(1ull << 22, 2ull * HELPERS * ncp);
   if (pool_cap > 0xffffffffull) return cudaErrorInvalidValue;  // list offsets are 32-bit
   if (ncp > IDX_MASK) return cudaErrorInvalidValue;               // heap entries hold 29-bit indices
   auto rnd = [](size_t n) { return (n + 255) / 256 * 256; };

@@ -1,17 +1,21 @@
-// warp_graph.cuh -- cancel_pairs and uncancel_pairs of msc_graph.cuh by one
-// warp.
+// warp_graph.cuh -- cancel_pairs and uncancel_pairs of msc_graph.cuh by warps.
 //
 // The order-dependent passes (the simplification's replay, the merges'
 // boundary steps) change the graph one pair at a time, and each change is a
 // handful of list edits whose cost is dependent memory round trips.  A pair's
 // edits all concern different lists (the neighbours' asc lists and des lists,
-// and a cell's lists hold cells of one dimension), so the warp makes them side
-// by side: up to 32 short lists (at most 8 runs, at most one added value) one
-// per lane, each read once into registers, edited there and written back; a
-// longer list by all lanes together, one merge for all added values and the
-// removed one.  Every list is left with the runs the
+// and a cell's lists hold cells of one dimension), so they are made side by
+// side: up to 32 short lists (at most 8 runs, at most one added value) by one
+// warp, a list per lane, each read once into registers, edited there and
+// written back; a longer list by all lanes of a warp together, one merge for
+// all added values and the removed one.  Every list is left with the runs the
 // one-thread functions leave, and the operation count (`ops`) grows by the
 // same amount.
+//
+// A cancellation is orient (which point's asc list holds the other), then
+// edit_neighbours by all warps of a team, and close; an uncancellation is
+// uncancel_list for each of its two lists, by one warp (uncancel_pairs) or as
+// tasks that a team's warps take (uncancel_shared).
 //
 // All lanes call every member function together with the same arguments and
 // hold the same copy of the graph's descriptor.
@@ -429,7 +433,7 @@ struct WarpGraph {
     G.tick(ticks);
   }
 
-  // One lane's share of cancel_pairs: list l of n runs (n <= N) takes the
+  // One lane's share of a cancellation: list l of n runs (n <= N) takes the
   // value ad (k = 1) with count mult * ad.y and loses r's run.
   template <int N>
   struct LaneEdit {
@@ -514,19 +518,6 @@ struct WarpGraph {
     return G.tick(warp_sum64(on ? E.ticks : 0ull));
   }
 
-  // cancelPairs (see Graph::cancel_pairs): false when the points are not connected
-  __device__ __forceinline__ bool cancel_pairs(uint32_t &cp0, uint32_t &cp1) {
-    Pair q{reinterpret_cast<const uint2 *>(G.L.off)[cp0], reinterpret_cast<const uint2 *>(G.L.off)[cp1],
-           reinterpret_cast<const uint2 *>(G.L.nrun)[cp0], reinterpret_cast<const uint2 *>(G.L.nrun)[cp1], cp0, cp1};
-    if (!orient(q)) return false;
-    cp0 = q.cp0;
-    cp1 = q.cp1;
-    edit_neighbours(q, 0, 1);
-    if (G.fail) return true;
-    close(q, 0);
-    __syncwarp();
-    return true;
-  }
   // A pair to cancel: both points' lists' places and lengths (asc, des).
   struct Pair {
     uint2 o0, o1, n0, n1;
