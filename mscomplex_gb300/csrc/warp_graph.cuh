@@ -51,18 +51,21 @@ struct TeamState {
   uint32_t fail, wrong;      // a pool, budget or wait ran out; a reference logic_error condition
   int lock;                  // 1: a warp uses the scratch all warps share
   uint32_t late;             // a wait on another warp ran out (fail is set too)
-  uint32_t beat;             // changes while any warp gets on with its work
+  uint32_t beat;             // parts done of lists that take long
   unsigned long long *shared_top;  // the pool's top where several blocks edit the graph (then top is unused)
 };
-// A wait on another warp ends after so many polls during which no warp of the
-// team got on.  (A list may take longer than that to rewrite: millions of
-// values are sorted by one warp in global memory, at worst by one lane.  Its
-// loops move the team's beat on at least every few ms.)
+// A wait on another warp polls so often, then looks whether the team got on
+// since the last time it looked: whether a task was taken, or the beat moved.
+// If neither, it gives up.  (A list may take longer than the polls to rewrite:
+// millions of values are sorted by one warp in global memory, at worst by one
+// lane.  Its loops count a beat at least every few ms; lists of usual lengths
+// have none.)  The look is outside the loop of the polls: within it, it took 5%
+// of the time of all uncancellations.
 #ifndef DMSC_WAIT_POLLS
 #define DMSC_WAIT_POLLS (1ull << 26)
 #endif
 constexpr unsigned long long WAIT_LIMIT = DMSC_WAIT_POLLS;
-constexpr uint32_t BEAT_STEPS = 4096;  // steps of a loop over a list between two beats (a power of two)
+constexpr uint32_t BEAT_STEPS = 4096;  // a loop over a list counts a beat after so many steps (a power of two)
 constexpr int BAR_EDIT = 3;
 
 struct WarpGraph {
@@ -80,26 +83,27 @@ struct WarpGraph {
   uint32_t nshared_stage = 0;
 
   __device__ __forceinline__ unsigned lt() const { return (1u << lane) - 1u; }
-  // the calling lane's warp has got on with its work
+  // by the calling lane: its warp has done a part of a long list
   __device__ __forceinline__ void moved_on() const {
     if (team) atomicAdd(&team->beat, 1u);
   }
-  // One more poll of a wait on another warp: whether to give up.  polls is 0
-  // before the first one; beat is the wait's own.
-  __device__ __forceinline__ bool give_up(unsigned long long &polls, uint32_t &beat) const {
-    if (*(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong) return true;
-    if (polls != 0 && polls < WAIT_LIMIT) {
-      ++polls;
+  // another warp's work has failed
+  __device__ __forceinline__ bool called_off() const {
+    return *(volatile uint32_t *)&team->fail || *(volatile uint32_t *)&team->wrong;
+  }
+  // All lanes, after a wait that was called off or whose polls ran out: whether
+  // to wait on, as the team got on since the last time (seen: what it had done
+  // then, ~0 the first time).
+  __device__ __forceinline__ bool wait_on(unsigned long long &seen) const {
+    uint32_t now = *(volatile uint32_t *)&team->beat - (uint32_t)*(volatile unsigned long long *)&team->ticket;  // (tasks count down)
+    now = __shfl_sync(FULL_WARP, now, 0);
+    if (__any_sync(FULL_WARP, called_off())) return false;
+    if (seen == now) {
+      if (lane == 0) *(volatile uint32_t *)&team->late = 1;
       return false;
     }
-    const uint32_t now = *(volatile uint32_t *)&team->beat;
-    if (polls != 0 && now == beat) {
-      *(volatile uint32_t *)&team->late = 1;
-      return true;
-    }
-    beat = now;
-    polls = 1;
-    return false;
+    seen = now;
+    return true;
   }
 
   // first run of p[0..n) (ascending values) with value >= x
@@ -665,14 +669,19 @@ struct WarpGraph {
     if (N <= room) {  // bitonic, padded to a power of two by values above every index
       for (unsigned long long i = n + lane; i < N; i += 32) b[i] = make_uint2(0xffffffffu, 0u);
       __syncwarp();
+      const bool counts = lane == 0 && N >= 4096;
       for (unsigned long long k = 2; k <= N; k <<= 1)
         for (unsigned long long j = k >> 1; j > 0; j >>= 1) {
+          if (counts) moved_on();
+          for (unsigned long long t = lane; t < N / 2;) {
+            const unsigned long long end = min(t + 32 * BEAT_STEPS, N / 2);
 #pragma unroll 4
-          for (unsigned long long t = lane; t < N / 2; t += 32) {
-            if ((t & (BEAT_STEPS * 32 - 1)) == 0) moved_on();  // (lane 0)
-            const unsigned long long i = 2 * t - (t & (j - 1)), o = i + j;  // the t-th pair at distance j
-            const uint2 x = b[i], y = b[o];
-            if ((x.x > y.x) == ((i & k) == 0)) { b[i] = y; b[o] = x; }
+            for (; t < end; t += 32) {
+              const unsigned long long i = 2 * t - (t & (j - 1)), o = i + j;  // the t-th pair at distance j
+              const uint2 x = b[i], y = b[o];
+              if ((x.x > y.x) == ((i & k) == 0)) { b[i] = y; b[o] = x; }
+            }
+            if (counts) moved_on();
           }
           __syncwarp();
         }
@@ -696,7 +705,7 @@ struct WarpGraph {
     auto is_head = [&](unsigned long long u) { return u < n && (u == 0 || b[u - 1].x != b[u].x); };
     uint32_t m = 0;
     for (unsigned long long u0 = 0; u0 < n; u0 += 32) {
-      if (lane == 0 && (u0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
+      if (lane == 0 && ((u0 + 32) & (32 * BEAT_STEPS - 1)) == 0) moved_on();
       m += __popc(__ballot_sync(FULL_WARP, is_head(u0 + lane)));
     }
     uint32_t off = G.L.off[l];
@@ -706,16 +715,17 @@ struct WarpGraph {
     bool bad = false;
     uint32_t w = 0;
     for (unsigned long long u0 = 0; u0 < n; u0 += 32) {
-      if (lane == 0 && (u0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
+      if (lane == 0 && ((u0 + 32) & (32 * BEAT_STEPS - 1)) == 0) moved_on();
       const unsigned long long u = u0 + lane;
       const bool head = is_head(u);
       const unsigned hb = __ballot_sync(FULL_WARP, head);
       if (head) {
         const uint32_t x = b[u].x;
         unsigned long long s = 0;
-        for (unsigned long long q = u; q < n && b[q].x == x; ++q) {
-          if ((q - u) % BEAT_STEPS == BEAT_STEPS - 1) moved_on();
-          s += b[q].y;
+        for (unsigned long long q = u; q < n && b[q].x == x;) {
+          const unsigned long long end = min(q + BEAT_STEPS, n);
+          for (; q < end && b[q].x == x; ++q) s += b[q].y;
+          if (q >= u + BEAT_STEPS) moved_on();
         }
         if (s > 0xffffffffull) bad = true;
         tot += s;
@@ -776,11 +786,9 @@ struct WarpGraph {
             cancelled = o <= turn;
             const uint32_t bit = 2 * (o - 1) + i;
             volatile const uint32_t *w = done + (bit >> 5);
-            unsigned long long polls = 0;
-            uint32_t beat = 0;
-            while (!cancelled && !((*w >> (bit & 31)) & 1u))
-              if (give_up(polls, beat)) {
-                t.stopped = true;  // the wait ran out, or another warp's pair failed
+            for (unsigned long long polls = 0; !cancelled && !((*w >> (bit & 31)) & 1u);)
+              if (++polls > WAIT_LIMIT || called_off()) {
+                t.stopped = true;  // the polls ran out, or another warp's pair failed
                 break;
               }
             __threadfence_block();
@@ -818,7 +826,7 @@ struct WarpGraph {
       const uint32_t sc = __shfl_sync(FULL_WARP, t.cnt, s), ss = __shfl_sync(FULL_WARP, t.src, s);
       const uint32_t so = __shfl_sync(FULL_WARP, o, s), sy = __shfl_sync(FULL_WARP, t.run.y, s);
       for (uint32_t q = lane; q < sc; q += 32) {
-        if ((q & (BEAT_STEPS * 32 - 1)) == 0) moved_on();  // (lane 0)
+        if (((q + 32) & (32 * BEAT_STEPS - 1)) == 0) moved_on();  // (lane 0)
         one(G.L.pool[ss + q], sy, so + q);
       }
     }
@@ -832,14 +840,17 @@ struct WarpGraph {
     if (stage && n <= nstage) return stage;
     if (team) {
       bool got = false;
-      if (lane == 0) {
-        unsigned long long polls = 0;
-        uint32_t beat = 0;
-        do got = atomicCAS(&team->lock, 0, 1) == 0;
-        while (!got && !give_up(polls, beat));
-        __threadfence_block();
+      for (unsigned long long seen = ~0ull;;) {
+        if (lane == 0)
+          for (unsigned long long polls = 0; !got && polls <= WAIT_LIMIT; ++polls) {
+            got = atomicCAS(&team->lock, 0, 1) == 0;
+            if (!got && called_off()) break;
+          }
+        got = __shfl_sync(FULL_WARP, got, 0);
+        if (got || !wait_on(seen)) break;
       }
-      if (!__shfl_sync(FULL_WARP, got, 0)) { G.fail = true; return nullptr; }
+      __threadfence_block();
+      if (!got) { G.fail = true; return nullptr; }
     }
     if (shared_stage && n <= nshared_stage) return shared_stage;
     if (n > G.tmp_cap) { drop_scratch(n); G.fail = true; return nullptr; }
@@ -877,9 +888,13 @@ struct WarpGraph {
     unsigned long long n = 0, ticks = 0;
     uint2 *b;
     if (nr <= 32) {  // one run per lane
-      const Item t = item_of(p, nr, lane, other, i, turn);
+      Item t;
+      for (unsigned long long seen = ~0ull;;) {
+        t = item_of(p, nr, lane, other, i, turn);
+        if (!__any_sync(FULL_WARP, t.stopped)) break;
+        if (!wait_on(seen)) { G.fail = true; return true; }
+      }
       if (!__any_sync(FULL_WARP, (uint32_t)lane < nr && t.run.x == other)) return false;  // "cancellable pair is not connected"
-      if (__any_sync(FULL_WARP, t.stopped)) { G.fail = true; return true; }
       if (__any_sync(FULL_WARP, t.wrong)) return false;
       if (!__any_sync(FULL_WARP, t.open)) {  // the list without the other point
         const unsigned keep = __ballot_sync(FULL_WARP, t.cnt != 0);
@@ -899,14 +914,17 @@ struct WarpGraph {
     } else {
       if (!holds(p, nr, other)) return false;
       for (uint32_t k0 = 0; k0 < nr; k0 += 32) {  // the items' number, and the checks
-        if (lane == 0 && (k0 & (BEAT_STEPS * 32 - 1)) == 0) moved_on();
-        const Item t = item_of(p, nr, k0 + lane, other, i, turn);
+        if (lane == 0 && ((k0 + 32) & (32 * BEAT_STEPS - 1)) == 0) moved_on();
+        Item t;
+        for (unsigned long long seen = ~0ull;;) {
+          t = item_of(p, nr, k0 + lane, other, i, turn);
+          if (!__any_sync(FULL_WARP, t.stopped)) break;
+          if (!wait_on(seen)) { G.fail = true; return true; }
+        }
         wrong |= t.wrong;
-        bad |= t.stopped;
         n += warp_sum64(t.cnt);
         ticks += warp_sum64(t.open ? 1ull + t.cnt : 0ull);
       }
-      if (__any_sync(FULL_WARP, bad)) { G.fail = true; return true; }
       if (__any_sync(FULL_WARP, wrong)) return false;
       if (!(b = take_scratch(n))) return true;
       uint2 *to = b;
@@ -940,10 +958,7 @@ struct WarpGraph {
       }
       __threadfence_block();
       __syncwarp();
-      if (lane == 0) {
-        atomicOr(&done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
-        moved_on();
-      }
+      if (lane == 0) atomicOr(&done[(2 * k + i) >> 5], 1u << ((2 * k + i) & 31));
     }
   }
 };
