@@ -567,7 +567,9 @@ __global__ void k_dc_write(DcArgs a, uint32_t n, const uint32_t *src) {
 }
 
 // ---------------------------------------------------------------------------
-// the boundary steps of a level, one block per job
+// the boundary steps of a level, all jobs in one launch: merge_up up to
+// UP_BLOCKS blocks per job (one where its cells go in plain order), merge_down
+// one block per job
 // ---------------------------------------------------------------------------
 enum SeqKind : int { SEQ_UP_CANCEL = 0, SEQ_DOWN_BOUNDARY = 1 };
 struct SeqJob {
@@ -1278,8 +1280,10 @@ double now_ms() {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// Runs the jobs (one block each) and brings the graphs' counters back; adds
-// its wall time to *ms.
+// Runs the jobs side by side and brings the graphs' counters back; adds its
+// wall time to *ms.  merge_up's blocks of one job take groups of cells from a
+// counter, share the list pool's top (an atomic, UpWork::top) and have a slice
+// of the graph's scratch per warp.
 cudaError_t run_seq(std::vector<MGraphHost *> &graphs, const std::vector<SeqJob> &jobs, uint32_t *status,
                     cudaStream_t st, double *ms) {
   if (jobs.empty()) return cudaSuccess;
@@ -1701,7 +1705,7 @@ cudaError_t merge_up_level_par(const std::vector<MergeJob> &jobs, unsigned long 
     cudaStreamSynchronize(st);
     return e;
   }
-  // the boundary cancellations, one block per merge, on mutable graphs
+  // the boundary cancellations, up to UP_BLOCKS blocks per merge, on mutable graphs
   std::vector<MGraphHost *> gp;
   std::vector<SeqJob> seq;
   for (int k = 0; k < nj; ++k) {

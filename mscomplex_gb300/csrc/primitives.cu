@@ -126,7 +126,7 @@ __device__ __forceinline__ void load4(const T *in, long long at, long long n, bo
 // block adds up the sums before its own and scans its chunk tile by tile (the
 // second read comes from L2 up to some 25 million items).  No block waits for
 // another: a single pass with decoupled look-back read the items once but
-// spent its time walking back over the tiles in flight (2^24 items: 57 us,
+// spent its time walking back over the tiles in flight (2^24 items: 68 us,
 // here 31; 8 bytes an item are 20 us).  A tile is 16 items a thread: each warp
 // owns 512 consecutive items in four rounds of 128, so that every load and
 // store instruction moves 512 consecutive bytes, and the next tile's loads are

@@ -1163,8 +1163,9 @@ cudaError_t simplify_batch_run(BatchSimplifyIO &io, cudaStream_t st) {
   if (e == cudaSuccess && ns) e = cudaMemcpyAsync(w->dargs, args.data(), sizeof(SimpArgs) * ns, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && ns) {
     // one grid per SM can keep 14 heap levels in shared memory; more grids
-    // than SMs keep 13, two per SM (measured on the 1000-grid workload: 13
-    // levels 108.8 ms, 12 levels (four per SM) 113.8, 14 levels 122.4)
+    // than SMs keep 13, two per SM (a batch of 1000 grids, two sets of inputs:
+    // 13 levels 46.0 and 53.1 ms, 12 levels (three per SM) 48.3 and 57.2, 14
+    // levels 55.1 and 44.1: it depends on which replay is the longest)
     const int levels = ns <= 152 ? TOP_LEVELS : TOP_LEVELS_BATCH;
     k_simp_meta<<<dim3(64, (unsigned)ns), 256, 0, st>>>(w->dargs);
     k_simp_prep<<<dim3(64, (unsigned)ns), 256, 0, st>>>(w->dargs);

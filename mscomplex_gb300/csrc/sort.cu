@@ -1,8 +1,10 @@
 // sort.cu -- stable LSD radix sort of (key, value) pairs of 32-bit words
 // (the reference's sort slot: BitonicSortProgram, dmsc/include/bitonic_sort.h).
 //
-// One pass over the keys counts the digits of all passes.  Each pass then
-// takes the pairs once: a block ranks a tile's pairs by their digit, learns
+// The scheme is the published single-pass one (Adinets and Merrill, "Onesweep",
+// 2022, after Merrill and Garland's decoupled look-back, 2016).  One pass over
+// the keys counts the digits of all passes.  Each pass then takes the pairs
+// once: a block ranks a tile's pairs by their digit, learns
 // how many pairs of each digit the earlier tiles hold by decoupled look-back
 // (tiles are taken from an atomic counter, so a block only waits for blocks
 // that already run), groups the tile by digit in shared memory, and writes
@@ -11,10 +13,11 @@
 // tiles in flight (256 words for each tile before a tile): for many pairs a tile
 // is as large as one block's registers and shared memory allow, one block per SM.
 // With 6,144 pairs a tile a pass over 3,000,017 took 41 us, with 20,480 31; a
-// histogram, a scan and a scatter of single pairs took 77 (a warp's 32 pairs
+// histogram, a scan and a scatter of single pairs took 75 (a warp's 32 pairs
 // went to 32 places).  Such tiles leave SMs idle and are long for fewer pairs: up to
 // 1.6 million the tiles have 4,096 (a call with 130,000 pairs 158 us with 20,480 a
-// tile, 90 so; 900,000: 165, 125; 1,500,000: 169, 154).  Up to 8,192 pairs are
+// tile, 90 so; 900,000: 165, 125; 1,500,000: 169, 154; they meet near 2 million, and
+// the line lies below, where the smaller tiles still gain a tenth).  Up to 8,192 pairs are
 // sorted by one block in one launch, 4 or 8 a thread (a call with 3,000 pairs 104
 // us with 20 a thread, 51 so; 6,000: 104, 61).
 #include "dmsc_common.cuh"
